@@ -429,6 +429,12 @@ __device__ __forceinline__ uint32_t depth_key(float d)
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// The depth of a key (+0 for either zero).
+__device__ __forceinline__ float key_depth(uint32_t k)
+{
+    return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
+}
+
 __device__ __forceinline__ float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
 // Shading arithmetic (not part of the bit-exact pipeline): fused
 // multiply-adds, one rounding each.

@@ -1241,7 +1241,8 @@ constexpr uint32_t kEmptyRegion = 16u | (16u << 10);  // lx0 = ly0 = 16 > lx1 = 
 template <bool MS = false>
 __device__ __forceinline__ void stage_tri(const PassArgs& a, uint32_t entry, uint32_t nr, uint32_t rank_base,
                                           int tileX, int tileY,
-                                          StagedTri& s, uint32_t& zkey, int* G = nullptr)
+                                          StagedTri& s, uint32_t& zkey, int* G = nullptr,
+                                          bool* wrapfree = nullptr)
 {
     const uint32_t ri = entry >> 2;
     if (ri >= nr)
@@ -1282,6 +1283,8 @@ __device__ __forceinline__ void stage_tri(const PassArgs& a, uint32_t entry, uin
     // where the centre is not), and the depth bound below holds at every
     // covered sample
     const bool wfree = wrap_free(t);
+    if (MS)
+        *wrapfree = wfree;
     const bool wf = !MS && wfree;
     int lx0 = 0, lx1 = 15, ly0 = 0, ly1 = 15;
     if (!accept)
@@ -1761,7 +1764,7 @@ __global__ void __launch_bounds__(kRasterThreads, MinBlocks) k_raster(PassArgs a
 // reads sample s as `const Vector2i& sampleOffset = MultiSampleOffsets[level]
 // [2 * s]` (Rasterizer.h:247, 382): the int goes through Vector2i's scalar
 // constructor, so the sample sits at (o, o) with o = table[level][2 s].
-__constant__ int kSampleOffsets[kMaxMsaaLog2 + 1][64] = {
+constexpr int kSampleOffsets[kMaxMsaaLog2 + 1][64] = {
     { 0, 0 },
     { 4, 4, -4, -4 },
     { -2, -6, 6, -2, -6, 2, 2, 6 },
@@ -1774,31 +1777,58 @@ __constant__ int kSampleOffsets[kMaxMsaaLog2 + 1][64] = {
       -2, 7, 0, -4, -2, -5, -7, 6, -8, 3, 4, -1, 2, 7, 4, -8 }
 };
 
-__device__ __forceinline__ int sample_offset(int level, int s) { return kSampleOffsets[level][2 * s]; }
-
-// Key of sample s (offset o) of staged triangle st at tile pixel (lx, ly):
-// FineRasterize_MultiSample / TrivialAcceptTriangle_MultiSample
-// (Rasterizer.h:202-300, 355-415): the biased pixel-centre edge values plus
-// o * G decide coverage (accepted entries skip the test), the barycentrics
-// and depth come from the unbiased values at the sample.
-__device__ __forceinline__ bool sample_key(const StagedTri& st, const int* G, int lx, int ly, int o, bool less,
-                                           uint64_t& key)
+// The offsets of samples 16 * half .. of a level, 4 bits each (offset + 8):
+// an immediate where the sample loop is unrolled, two shifts where it is not,
+// instead of a constant-memory load per sample.
+constexpr unsigned long long sample_pack(int level, int half)
 {
-    // (no early exit: lanes of a warp test different samples, and the
-    // arithmetic of an uncovered one costs the warp nothing extra)
-    const uint32_t fl = st.flags;
-    const int l1 = wadd(wadd(wadd(wmul(st.A1, lx), wmul(st.D1, ly)), st.K1), wmul(o, G[1]));
-    const int l2 = wadd(wadd(wadd(wmul(st.A2, lx), wmul(st.D2, ly)), st.K2), wmul(o, G[2]));
-    const int e0 = wadd(wadd(wadd(wmul(st.A0, lx), wmul(st.D0, ly)), st.K0), wmul(o, G[0]));
-    const int e1 = wadd(l1, (fl & (1u << 21)) ? -1 : 0);
-    const int e2 = wadd(l2, (fl & (1u << 22)) ? -1 : 0);
-    const bool inside = (fl & (1u << 20)) || (e0 | e1 | e2) >= 0;
-    const float L0 = fmul(__int2float_rn(l1), st.invDet);
-    const float L1 = fmul(__int2float_rn(l2), st.invDet);
-    const float L2 = fsub(fsub(1.0f, L0), L1);
-    const float d = fadd(fadd(fmul(L0, st.z0), fmul(L1, st.z1)), fmul(L2, st.z2));
-    key = ((uint64_t)depth_key(d) << 32) | (less ? st.rank : ~st.rank);
-    return inside && d == d;
+    unsigned long long bits = 0;
+    for (int s = 0; s < 16 && 16 * half + s < (1 << level); s++)
+        bits |= (unsigned long long)(kSampleOffsets[level][2 * (16 * half + s)] + 8) << (4 * s);
+    return bits;
+}
+constexpr int log2_of(int S) { return S <= 1 ? 0 : 1 + log2_of(S / 2); }
+
+template <int S>
+struct SamplePack
+{
+    static constexpr unsigned long long lo = sample_pack(log2_of(S), 0), hi = sample_pack(log2_of(S), 1);
+};
+
+template <int S>
+__device__ __forceinline__ int sample_offset(int s)
+{
+    return (int)(((s < 16 ? SamplePack<S>::lo : SamplePack<S>::hi) >> (4 * (s & 15))) & 15u) - 8;
+}
+
+// A staged entry with several samples: the fields of StagedTri, the change G
+// of each edge per 1/16 pixel along the diagonal the samples sit on, and Q,
+// the edge constants raised to the largest value any sample of a pixel can
+// see.  112 bytes: 16-byte loads of eight consecutive entries hit eight
+// different bank groups.
+struct __align__(16) StagedMs
+{
+    int A0, D0, Q0, A1;
+    int D1, Q1, A2, D2;
+    int Q2;
+    uint32_t flags, rank;
+    int K0;
+    int K1, K2, G0, G1;
+    int G2;
+    float invDet, z0, z1;
+    float z2;
+    uint32_t pad[7];
+};
+static_assert(sizeof(StagedMs) == 112, "odd multiple of 16 bytes");
+
+// Can any sample of pixel (lx, ly) be covered?  (Always, flag bit 23, where
+// the entry is accepted whole or its edge values can wrap.)
+__device__ __forceinline__ bool pixel_possible(const StagedMs& st, int lx, int ly)
+{
+    const int q0 = wadd(wadd(wmul(st.A0, lx), wmul(st.D0, ly)), st.Q0);
+    const int q1 = wadd(wadd(wmul(st.A1, lx), wmul(st.D1, ly)), st.Q1);
+    const int q2 = wadd(wadd(wmul(st.A2, lx), wmul(st.D2, ly)), st.Q2);
+    return (st.flags & (1u << 23)) || (q0 | q1 | q2) >= 0;
 }
 
 // Float -> 8 bits as Color4b::FromFloats: clamp, scale by 255, round half up.
@@ -1814,89 +1844,138 @@ __device__ __forceinline__ uint32_t to_byte(float v)
 // (FrameBuffer::Resolve, FrameBuffer.cpp:70-87): each sample stores its
 // winner's colour shaded at the pixel centre as 8 bits (Renderer.cpp:
 // 295-350), the samples are averaged in float (alpha 1 per covered sample,
-// 0 for the clear value).  Samples that share a winner share its shading.
-// The winners come from the pixel's keys (key[s * 256], shared memory), read
-// sample by sample.  Common: the per-vertex-attribute shaders, inline (no
-// call); otherwise shade_fragment (the FP64 and textured shaders out of line).
-template <bool Common>
+// 0 for the clear value).
+// The pixel's keys (key[s * 256], shared memory) are worked off winner by
+// winner: the first open sample's winner is shaded, then every sample it wins
+// is written and its 8-bit colour left in the key's low word for the average
+// in sample order.  A warp so runs the shading once per distinct winner of
+// its busiest pixel (one to three) instead of once per sample at which any of
+// its pixels changes winner: 8 samples of the sphere at 1280x720, 94 -> 72 us.
+// The depth comes out of the key.  Common: the per-vertex-attribute shaders,
+// inline (no call); otherwise shade_fragment (the FP64 and textured shaders
+// out of line).
+template <int S, bool Common>
 static __device__ __forceinline__ void write_pixel_ms(const PassArgs& a, const FrameDesc& f,
-                                                   const unsigned long long* key, bool less, uint32_t nr, int S,
+                                                   unsigned long long* key, bool less, uint32_t nr,
                                                    uint64_t pix, int px, int py)
 {
-    const int level = a.msaa_log2;
     const uint64_t plane = a.total_pixels;
-    float acc[4] = { 0.f, 0.f, 0.f, 0.f };
-    uint32_t last = kNoTriangle;
-    float cf[3] = { 0.f, 0.f, 0.f };  // the winner's 8-bit colour / 255
-    RTri t;                            // the record of `last`
-    for (int s = 0; s < S; s++)
+    uint32_t* low_words = reinterpret_cast<uint32_t*>(key);  // sample s: words 512 s (rank term), 512 s + 1 (depth)
+    uint32_t todo = S == 32 ? 0xFFFFFFFFu : (1u << (S & 31)) - 1u, covered = 0;
+    while (todo)
     {
-        const uint32_t low = (uint32_t)key[s * 256];
-        const uint32_t r = raster_triangle_of(a, less ? low : ~low, nr);
-        if (r == kNoTriangle)
+        // the next sample's winner, shaded once for every sample it wins
+        const uint32_t low = low_words[512 * (__ffs(todo) - 1)];
+        const uint32_t ri = raster_triangle_of(a, less ? low : ~low, nr);
+        uint32_t id = kNoTriangle, rgb = 0;
+        if (ri != kNoTriangle)
         {
-            a.depth[s * plane + pix] = 1.0f;
-            a.tri_id[s * plane + pix] = kNoTriangle;
-            continue;
-        }
-        if (r != last)
-        {
-            t = a.rtris[r];
+            const RTri t = a.rtris[ri];
+            id = t.order >> 4;
             float L0, L1;
             depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
             const float3 c = Common ? shade_common(f, t, a.polys, L0, L1)
-                                    : shade_fragment(f, t, a.rtris + r, a.polys, L0, L1, px, py);
-            cf[0] = fdiv((float)to_byte(c.x), 255.0f);
-            cf[1] = fdiv((float)to_byte(c.y), 255.0f);
-            cf[2] = fdiv((float)to_byte(c.z), 255.0f);
-            last = r;
+                                    : shade_fragment(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
+            rgb = to_byte(c.x) | (to_byte(c.y) << 8) | (to_byte(c.z) << 16);
         }
-        const int o = sample_offset(level, s);
-        float L0, L1;
-        a.depth[s * plane + pix] = depth_at(t, (px << 4) + 8 + o, (py << 4) + 8 + o, L0, L1);
-        a.tri_id[s * plane + pix] = t.order >> 4;
+#pragma unroll (S <= 8 ? S : 4)
+        for (int s = 0; s < S; s++)
+        {
+            if (!((todo >> s) & 1u) || low_words[512 * s] != low)
+                continue;
+            todo &= ~(1u << s);
+            float d = 1.0f;
+            if (ri != kNoTriangle)
+            {
+                covered |= 1u << s;
+                low_words[512 * s] = rgb;
+                d = key_depth(low_words[512 * s + 1]);
+                if (d == 0.0f)
+                {
+                    // the key does not keep the sign of a zero
+                    const int o = sample_offset<S>(s);
+                    float L0, L1;
+                    d = depth_at(a.rtris[ri], (px << 4) + 8 + o, (py << 4) + 8 + o, L0, L1);
+                }
+            }
+            a.depth[s * plane + pix] = d;
+            a.tri_id[s * plane + pix] = id;
+        }
+    }
+    // the samples' 8-bit colours, averaged in sample order
+    float acc[3] = { 0.f, 0.f, 0.f }, cf[3] = { 0.f, 0.f, 0.f };
+    uint32_t last = 0;
+#pragma unroll 1
+    for (uint32_t m = covered; m; m &= m - 1u)
+    {
+        const uint32_t rgb = low_words[512 * (__ffs(m) - 1)];
+        if (rgb != last)
+        {
+            last = rgb;
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+                cf[q] = fdiv((float)((rgb >> (8 * q)) & 255u), 255.0f);
+        }
 #pragma unroll
         for (int q = 0; q < 3; q++)
             acc[q] = fadd(acc[q], cf[q]);
-        acc[3] = fadd(acc[3], 1.0f);
     }
     const float inv = fdiv(1.0f, (float)S);
-    a.color[pix] = make_float4(fmul(acc[0], inv), fmul(acc[1], inv), fmul(acc[2], inv), fmul(acc[3], inv));
+    a.color[pix] = make_float4(fmul(acc[0], inv), fmul(acc[1], inv), fmul(acc[2], inv),
+                               fmul((float)__popc(covered), inv));
 }
 
 // A multisampled tile shaded by the FP64 or the textured shader: out of line,
 // so that the common shaders' loop keeps its registers.  (`a` is the
 // kernel's grid-constant parameter: passed by address, it is not copied.)
+template <int S>
 static __device__ __noinline__ void shade_tile_ms_slow(const PassArgs& a, const FrameDesc& f,
-                                                       const unsigned long long* key, int tileX, int tileY, bool less,
-                                                       uint32_t nr, int S)
+                                                       unsigned long long* key, int first, int step, int tileX,
+                                                       int tileY, bool less, uint32_t nr)
 {
-    const uint32_t lane = threadIdx.x & 31;
 #pragma unroll 1
-    for (int k = 0; k < 8; k++)
+    for (int p = first; p < 256; p += step)
     {
-        const int p = (int)lane + 32 * k;
         const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
         if (px >= f.width || py >= f.height)
             continue;
-        write_pixel_ms<false>(a, f, key + p, less, nr, S, f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px,
-                              px, py);
+        write_pixel_ms<S, false>(a, f, key + p, less, nr, f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px,
+                                 px, py);
     }
 }
 
-// Raster with S samples per pixel: persistent warps on the same work items
-// as k_raster, keys [sample][pixel] in dynamic shared memory, every entry's
-// (entry, pixel) pairs spread over the lanes with a loop over the samples,
-// entries behind the tile's samples skipped.  Split tiles merge per sample
-// in the key buffer (S planes).
+// Raster with S samples per pixel: persistent blocks on the same work items as
+// k_raster.  A block's W warps share one tile and its keys [sample][pixel] in
+// dynamic shared memory: with a tile per warp the keys (2 KiB per sample) left
+// room for 12 warps per SM at 8 samples and 3 at 32, and a tile's chain of
+// dependent loads and tests ran on one warp (7.8 % of the warps active on the
+// sphere at 8 samples).  Each warp stages its own chunks of 32 entries; their
+// (entry, pixel) pairs are spread over the lanes, the pixels where no sample
+// can be covered are dropped by one conservative test, and the rest are queued
+// and take the S samples 32 pixels at a time.  Entries behind the tile's
+// samples are skipped.  Split tiles merge per sample in the key buffer (S
+// planes).
+// Raster and shading, a warp per tile -> a block per tile: terrain of 2,097,152
+// triangles at 1920x1080, 4 samples 350-364 -> 270 us, 8 samples 702 -> 373;
+// sphere at 1280x720, 4 samples 88 -> 55, 8 samples 139 -> 72; 512x512-quad
+// terrain at 1280x720, 16 samples 1104 -> 317, 32 samples 3146 -> 717.
+// W and the blocks per SM (registers a thread): 4 warps at 8 blocks (64, some
+// spilled) against 5 (96, none) measured 270 and 313 us on the terrain at 4
+// samples, 55 and 51 on the sphere; 2 warps 291 and 59, 8 warps 350 and 61.
+// With 16 and 32 samples the keys allow 3 to 5 blocks: 8 warps each.
+constexpr int kMsWarpBytes = 32 * (int)sizeof(StagedMs) + 64 * 2;
 
-// Blocks of 4 warps (2 with 16 samples, 1 with 32); registers capped where
-// shared memory lets 5 blocks share an SM (2 and 4 samples: 96 registers a
-// thread), the compiler's choice where it lets 3.
+__host__ __device__ constexpr int ms_warps(int S) { return S <= 8 ? 4 : 8; }
+__host__ __device__ constexpr int ms_blocks(int S) { return S <= 8 ? 8 : 3; }
+
 template <int S>
-__global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_constant__ PassArgs a)
+__global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(const __grid_constant__ PassArgs a)
 {
+    constexpr int W = ms_warps(S);
+    constexpr int kThreads = 32 * W;
+    constexpr int kPixels = 256 / kThreads;
     extern __shared__ unsigned long long ms_shared[];
+    __shared__ uint32_t s_next, s_done, s_bound[W];
     if (*(volatile uint32_t*)&a.status->error)
         return;  // the pass failed (see k_bin_move); every thread of the block leaves
     // ceil(65536 / w): ((p * s_recip[w]) >> 16) == p / w for 0 <= p < 256
@@ -1906,20 +1985,25 @@ __global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_
         s_recip[threadIdx.x] = (65536u + threadIdx.x - 1u) / threadIdx.x;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long* key = ms_shared + (size_t)warp * (256 * S + 32 * 10);
-    StagedTri* staged = reinterpret_cast<StagedTri*>(key + 256 * S);            // 32 x 64 bytes
-    int* sg = reinterpret_cast<int*>(key + 256 * S + 32 * 8);                    // 32 x 3 ints (G)
-    const int level = a.msaa_log2;
+    unsigned long long* key = ms_shared;
+    unsigned char* mine = reinterpret_cast<unsigned char*>(ms_shared + 256 * S) + warp * kMsWarpBytes;
+    StagedMs* staged = reinterpret_cast<StagedMs*>(mine);
+    uint16_t* queue = reinterpret_cast<uint16_t*>(mine + 32 * sizeof(StagedMs));  // up to 63 pixels
     // raster-triangle slots in use: one per input triangle, then the fan pieces
     const uint32_t nr = (uint32_t)min((uint64_t)a.total_tris + *(volatile uint32_t*)&a.counters[0],
                                       (uint64_t)a.rtri_capacity);
     const uint32_t nheavy = *(volatile uint32_t*)&a.counters[6];
     const uint32_t nitems = (uint32_t)min((uint64_t)nheavy + *(volatile uint32_t*)&a.counters[7], a.item_capacity);
     const uint64_t plane = a.total_pixels;
-    // each warp's first item is its own (the heaviest ones, no claim), the
+    auto next_item = [&]() -> uint32_t {
+        if (threadIdx.x == 0)
+            s_next = gridDim.x + atomicAdd(&a.counters[3], 1u);
+        __syncthreads();
+        return s_next;
+    };
+    // each block's first item is its own (the heaviest ones, no claim), the
     // rest are claimed one at a time
-    for (uint32_t q = blockIdx.x * (blockDim.x >> 5) + warp; q < nitems;
-         q = claim_item(a, gridDim.x * (blockDim.x >> 5)))
+    for (uint32_t q = blockIdx.x; q < nitems; q = next_item())
     {
         const uint4 item = a.items[q < nheavy ? q : (uint32_t)(a.item_capacity - 1 - (q - nheavy))];
         const uint32_t tile = item.x & ~kSplitTile;
@@ -1944,21 +2028,25 @@ __global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_
             if (split && e0 == e1)
             {
                 if (item.y != bin0 || kept != 0)
+                {
+                    __syncthreads();
                     continue;  // the tile's kept entries are in its other items
+                }
                 split = false;  // it kept none: its first item writes the background
             }
         }
         if (e0 == e1 && !split)
         {
             // a tile with no bin entry: its background, with no key
-            for (int k = 0; k < 8; k++)
+            for (int k = 0; k < kPixels; k++)
             {
-                const int p = (int)lane + 32 * k;
+                const int p = (int)threadIdx.x + kThreads * k;
                 const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
                 if (px < f.width && py < f.height)
                 {
                     const uint64_t pix = f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px;
                     a.color[pix] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
                     for (int s = 0; s < S; s++)
                     {
                         a.depth[s * plane + pix] = 1.0f;
@@ -1966,18 +2054,56 @@ __global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_
                     }
                 }
             }
+            __syncthreads();
             continue;
         }
         const unsigned long long clear = ((unsigned long long)0xBF800000u << 32) | (less ? 0u : 0xFFFFFFFFu);
-        for (int k = (int)lane; k < 256 * S; k += 32)
+        for (int k = (int)threadIdx.x; k < 256 * S; k += kThreads)
             key[k] = clear;
-        __syncwarp();
+        if (lane == 0)
+            s_bound[warp] = 0xFFFFFFFFu;
+        __syncthreads();
 
         // depth bound of the tile: the nearest triangle that covers it whole
         // (every sample), then the largest depth key of its samples so far
         const uint32_t tzocc = min(0xBF800000u, a.tile_zocc[tile]);
         uint32_t tzmax = tzocc;
-        for (uint32_t c = e0; c < e1; c += 32)
+        // one queued pixel: entry << 8 | pixel of the tile, its samples tested
+        auto test_samples = [&](uint32_t e) {
+            const StagedMs& st = staged[e >> 8];
+            const int p = (int)(e & 255u), x = p & 15, y = p >> 4;
+            const uint32_t fl = st.flags;
+            const int c0 = wadd(wadd(wmul(st.A0, x), wmul(st.D0, y)), st.K0);
+            const int c1 = wadd(wadd(wmul(st.A1, x), wmul(st.D1, y)), st.K1);
+            const int c2 = wadd(wadd(wmul(st.A2, x), wmul(st.D2, y)), st.K2);
+            const int b1 = (fl & (1u << 21)) ? -1 : 0, b2 = (fl & (1u << 22)) ? -1 : 0;
+            const bool accept = (fl & (1u << 20)) != 0;
+            const uint32_t rank = less ? st.rank : ~st.rank;
+            const int G0 = st.G0, G1 = st.G1, G2 = st.G2;
+            const float invDet = st.invDet, z0 = st.z0, z1 = st.z1, z2 = st.z2;
+#pragma unroll (S <= 8 ? S : 8)
+            for (int s = 0; s < S; s++)
+            {
+                // FineRasterize_MultiSample / TrivialAcceptTriangle_MultiSample
+                // (Rasterizer.h:202-300, 355-415): the biased pixel-centre
+                // edge values plus o * G decide coverage (accepted entries
+                // skip the test), the barycentrics and depth come from the
+                // unbiased values at the sample
+                const int o = sample_offset<S>(s);
+                const int e0 = wadd(c0, wmul(o, G0)), l1 = wadd(c1, wmul(o, G1)), l2 = wadd(c2, wmul(o, G2));
+                const bool inside = accept || (e0 | wadd(l1, b1) | wadd(l2, b2)) >= 0;
+                const float L0 = fmul(__int2float_rn(l1), invDet);
+                const float L1 = fmul(__int2float_rn(l2), invDet);
+                const float L2 = fsub(fsub(1.0f, L0), L1);
+                const float d = fadd(fadd(fmul(L0, z0), fmul(L1, z1)), fmul(L2, z2));
+                const unsigned long long k = ((uint64_t)depth_key(d) << 32) | rank;
+                unsigned long long* slot = &key[s * 256 + p];
+                const unsigned long long cur = *slot;
+                if (inside && d == d && k < cur)
+                    atomicMin(slot, k);
+            }
+        };
+        for (uint32_t c = e0 + 32 * warp; c < e1; c += kThreads)
         {
             const uint32_t m = min(32u, e1 - c);
             int area = 0;
@@ -1986,21 +2112,30 @@ __global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_
                 StagedTri st;
                 uint32_t zk;
                 int G[3];
-                stage_tri<true>(a, a.bins[c + lane], nr, f.tri_base << 4, tileX, tileY, st, zk, G);
+                bool wfree = false;
+                stage_tri<true>(a, a.bins[c + lane], nr, f.tri_base << 4, tileX, tileY, st, zk, G, &wfree);
                 const uint32_t fl = st.flags;
                 const int rx0 = fl & 31, rx1 = (fl >> 5) & 31, ry0 = (fl >> 10) & 31, ry1 = (fl >> 15) & 31;
                 if (zk <= tzmax && rx0 <= rx1 && ry0 <= ry1)
                 {
-                    staged[lane] = st;
-                    sg[3 * lane] = G[0];
-                    sg[3 * lane + 1] = G[1];
-                    sg[3 * lane + 2] = G[2];
+                    StagedMs& t = staged[lane];
+                    t.A0 = st.A0; t.D0 = st.D0; t.A1 = st.A1; t.D1 = st.D1; t.A2 = st.A2; t.D2 = st.D2;
+                    t.K0 = st.K0; t.K1 = st.K1; t.K2 = st.K2;
+                    t.G0 = G[0]; t.G1 = G[1]; t.G2 = G[2];
+                    // the largest o * G over the offsets [-8, 7] of any sample table
+                    t.Q0 = wadd(st.K0, G[0] > 0 ? wmul(7, G[0]) : wmul(-8, G[0]));
+                    t.Q1 = wadd(st.K1, G[1] > 0 ? wmul(7, G[1]) : wmul(-8, G[1]));
+                    t.Q2 = wadd(st.K2, G[2] > 0 ? wmul(7, G[2]) : wmul(-8, G[2]));
+                    t.flags = fl | ((fl & (1u << 20)) || !wfree ? (1u << 23) : 0u);
+                    t.rank = st.rank;
+                    t.invDet = st.invDet; t.z0 = st.z0; t.z1 = st.z1; t.z2 = st.z2;
                     area = (rx1 - rx0 + 1) * (ry1 - ry0 + 1);
                 }
             }
             // (entry, pixel) pairs numbered across the warp and taken 32 at a
-            // time, each lane testing the S samples of its pixel, so lanes do
-            // not idle on entries of a few pixels
+            // time, so lanes do not idle on entries of a few pixels; pixels
+            // with a sample that may be covered are queued and, 32 at a time
+            // again, their S samples tested
             int incl = area;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1)
@@ -2010,6 +2145,7 @@ __global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_
             }
             const int pairs = __shfl_sync(0xffffffffu, incl, 31);
             __syncwarp();
+            int queued = 0;
             for (int base = 0; base < pairs; base += 32)
             {
                 const int p = base + (int)lane;
@@ -2022,41 +2158,58 @@ __global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_
                     if (v <= p) j += st;
                 }
                 const int first = __shfl_sync(0xffffffffu, incl - area, j);
+                bool keep = false;
+                uint32_t e = 0;
                 if (p < pairs)
                 {
-                    const StagedTri st = staged[j];
-                    const int G[3] = { sg[3 * j], sg[3 * j + 1], sg[3 * j + 2] };
+                    const StagedMs& st = staged[j];
                     const uint32_t fl = st.flags;
                     const int rx0 = fl & 31, rx1 = (fl >> 5) & 31, ry0 = (fl >> 10) & 31;
                     const int rw = rx1 - rx0 + 1, local = p - first;
                     const int dy = (int)(((uint32_t)local * s_recip[rw]) >> 16);
                     const int x = rx0 + local - dy * rw, y = ry0 + dy;
-#pragma unroll 4
-                    for (int s = 0; s < S; s++)
-                    {
-                        uint64_t k;
-                        unsigned long long* slot = &key[s * 256 + y * 16 + x];
-                        const bool hit = sample_key(st, G, x, y, sample_offset(level, s), less, k);
-                        const unsigned long long cur = *slot;
-                        if (hit && k < cur)
-                            atomicMin(slot, (unsigned long long)k);
-                    }
+                    e = ((uint32_t)j << 8) | (uint32_t)(y * 16 + x);
+                    keep = pixel_possible(st, x, y);
+                }
+                const uint32_t kept_lanes = __ballot_sync(0xffffffffu, keep);
+                if (keep)
+                    queue[queued + __popc(kept_lanes & ((1u << lane) - 1u))] = (uint16_t)e;
+                queued += __popc(kept_lanes);
+                __syncwarp();
+                if (queued >= 32)
+                {
+                    queued -= 32;
+                    test_samples(queue[queued + lane]);
+                    __syncwarp();
                 }
             }
+            if ((int)lane < queued)
+                test_samples(queue[lane]);
             __syncwarp();
-            if (c + 32 < e1)
+            if (c + kThreads < e1)
             {
+                // each warp takes the bound of its share of the keys again
+                // and combines it with the others' last ones (keys only fall:
+                // an old bound is a valid, larger one)
                 uint32_t mz = 0;
-                for (int k = (int)lane; k < 256 * S; k += 32)
+                for (int k = (int)threadIdx.x; k < 256 * S; k += kThreads)
                     mz = max(mz, (uint32_t)(key[k] >> 32));
-                tzmax = min(tzocc, __reduce_max_sync(0xffffffffu, mz));
+                mz = __reduce_max_sync(0xffffffffu, mz);
+                if (lane == 0)
+                    *(volatile uint32_t*)&s_bound[warp] = mz;
+                __syncwarp();
+#pragma unroll
+                for (int w = 0; w < W; w++)
+                    mz = max(mz, *(volatile uint32_t*)&s_bound[w]);
+                tzmax = min(tzocc, mz);
             }
         }
+        __syncthreads();
 
         bool shade = true;
         if (split)
         {
-            for (int k = (int)lane; k < 256 * S; k += 32)
+            for (int k = (int)threadIdx.x; k < 256 * S; k += kThreads)
             {
                 const int s = k >> 8, p = k & 255;
                 const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
@@ -2065,15 +2218,14 @@ __global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_
                     atomicMax(&a.keybuf[s * plane + f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px], ~kk);
             }
             // acquire-release count, as in k_raster
-            __syncwarp();
-            uint32_t done = 0;
-            if (lane == 0)
-                done = atomic_add_acq_rel(&a.tile_count[tile], e1 - e0) + (e1 - e0);
-            shade = __shfl_sync(0xffffffffu, done, 0) == kept;
-            __syncwarp();  // lane 0's acquire, then every lane's reads
+            __syncthreads();
+            if (threadIdx.x == 0)
+                s_done = atomic_add_acq_rel(&a.tile_count[tile], e1 - e0) + (e1 - e0);
+            __syncthreads();
+            shade = *(volatile uint32_t*)&s_done == kept;
             if (shade)
             {
-                for (int k = (int)lane; k < 256 * S; k += 32)
+                for (int k = (int)threadIdx.x; k < 256 * S; k += kThreads)
                 {
                     const int s = k >> 8, p = k & 255;
                     const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
@@ -2084,31 +2236,28 @@ __global__ void __launch_bounds__(128, S <= 4 ? 5 : 3) k_raster_ms(const __grid_
                         key[k] = m ? ~m : clear;
                     }
                 }
-                __syncwarp();
+                __syncthreads();
             }
         }
         if (shade && (f.ps_kind == 1 || f.ps_kind == 4))
-            shade_tile_ms_slow(a, f, key, tileX, tileY, less, nr, S);
+            shade_tile_ms_slow<S>(a, f, key, (int)threadIdx.x, kThreads, tileX, tileY, less, nr);
         else if (shade)
         {
 #pragma unroll 1
-            for (int k = 0; k < 8; k++)
+            for (int p = (int)threadIdx.x; p < 256; p += kThreads)
             {
-                const int p = (int)lane + 32 * k;
                 const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
                 if (px >= f.width || py >= f.height)
                     continue;
-                write_pixel_ms<true>(a, f, key + p, less, nr, S,
-                                     f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px, px, py);
+                write_pixel_ms<S, true>(a, f, key + p, less, nr,
+                                        f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px, px, py);
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
-// Warps per block and dynamic shared memory of k_raster_ms with S samples.
-static int ms_warps(int S) { return S <= 8 ? 4 : (S == 16 ? 2 : 1); }
-static size_t ms_smem(int S) { return (size_t)ms_warps(S) * (256 * S + 32 * 10) * sizeof(unsigned long long); }
+static size_t ms_smem(int S) { return (size_t)256 * S * sizeof(unsigned long long) + (size_t)ms_warps(S) * kMsWarpBytes; }
 
 // -------------------------------------------------------------------------
 // Renderer::GetBackBuffer compatibility: RGBA8, bottom-up (FrameBuffer.cpp:41).
@@ -2211,8 +2360,14 @@ Tuning default_tuning()
     return t;
 }
 
-cudaError_t launch_pipeline(const PassArgs& a, cudaStream_t s, cudaEvent_t* ev)
+cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* ev)
 {
+    PassArgs a = pass;
+    // With several samples a block of warps shares an item, so an item takes
+    // more entries (twice, four times with 8 warps): 4 samples of the terrain
+    // 309 -> 303 us, 16 samples 381 -> 317.
+    if (a.msaa_log2 > 0)
+        a.tune.item_entries = min(1024, a.tune.item_entries * (a.msaa_log2 <= 3 ? 2 : 4));
     const int sms = a.num_sms > 0 ? a.num_sms : 148;
     const uint32_t nscan = scan_blocks(a.total_tiles);
     auto mark = [&](int i) {
