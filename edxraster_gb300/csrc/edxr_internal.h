@@ -143,7 +143,7 @@ struct DeviceStatus
 struct Tuning
 {
     int small_region;     // bin entries whose pixel region is at most this are rasterized triangle-parallel
-    int raster_variant;   // 0/1: k_raster with the triangle-parallel path (3 / 5 blocks per SM), 2: pixel-parallel only
+    int raster_variant;   // 0/1: k_raster with the triangle-parallel path, 2: pixel-parallel only
     int bin_blocks_per_sm;
     int raster_blocks_per_sm;  // 0 = as many as fit
     int item_entries;     // bin entries per raster work item; items of at least 3/4 of it are handed out first

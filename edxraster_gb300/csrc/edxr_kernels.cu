@@ -1509,8 +1509,13 @@ static __device__ __noinline__ void shade_tile_slow(const PixelOut out, const Fr
     }
 }
 
-template <int MinBlocks, bool SmallPath>
-__global__ void __launch_bounds__(kRasterThreads, MinBlocks) k_raster(PassArgs a)
+// 3 blocks per SM: the 80 registers a thread hold the shading without spills.
+// At 5 blocks (48 registers, 156 bytes spilled) the raster stage took 119
+// instead of 100 us on the terrain (2,097,152 triangles, 1920x1080), 235
+// instead of 217 on the binning stress (3840x2160), 67 instead of 55 on a
+// 301x301-quad terrain at 1366x769; at 4 blocks 109, 219 and 61; at 2 blocks
+// (124 registers) 111, 250 and 53.
+__global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
 {
     __shared__ unsigned long long s_key[kRasterWarps][256];
     __shared__ StagedSlot s_tri[kRasterWarps][32];
@@ -1613,7 +1618,7 @@ __global__ void __launch_bounds__(kRasterThreads, MinBlocks) k_raster(PassArgs a
                 {
                     staged[lane].s = s;
                     const int area = (rx1 - rx0 + 1) * (ry1 - ry0 + 1);
-                    if (SmallPath && !(fl & (1u << 20)) && area <= small_region)
+                    if (!(fl & (1u << 20)) && area <= small_region)
                         nsmall = area;
                     else
                         big = true;
@@ -2276,31 +2281,23 @@ __global__ void k_back_buffer(const float4* color, uchar4* out, int width, int h
 
 // -------------------------------------------------------------------------
 
-// Raster variants: 0 and 1 carry the triangle-parallel path (3 blocks per SM,
-// whose 85 registers a thread hold the shading epilogue without spills / 5
-// blocks per SM); 2 is pixel-parallel only, capped for 6.
-static int raster_occupancy(int variant)
+// Resident blocks per SM of k_raster.
+static int raster_occupancy()
 {
-    static int per_sm[3] = { 0, 0, 0 };
-    if (!per_sm[variant])
+    static int per_sm = 0;
+    if (!per_sm)
     {
-        cudaError_t e;
-        if (variant == 0)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_raster<3, true>, kRasterThreads, 0);
-        else if (variant == 1)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_raster<5, true>, kRasterThreads, 0);
-        else
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[2], k_raster<6, false>, kRasterThreads, 0);
-        if (e != cudaSuccess || per_sm[variant] < 1)
-            per_sm[variant] = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_raster, kRasterThreads, 0) != cudaSuccess || n < 1)
+            n = 1;
+        per_sm = n;
     }
-    return per_sm[variant];
+    return per_sm;
 }
 
 static int raster_blocks(int sms, const Tuning& t)
 {
-    const int variant = (t.raster_variant >= 0 && t.raster_variant <= 2) ? t.raster_variant : 1;
-    int per = raster_occupancy(variant);
+    int per = raster_occupancy();
     if (t.raster_blocks_per_sm > 0 && t.raster_blocks_per_sm < per)
         per = t.raster_blocks_per_sm;
     return sms * per;
@@ -2340,9 +2337,7 @@ static int ms_occupancy(int level)
 
 void prepare_kernels()
 {
-    raster_occupancy(0);
-    raster_occupancy(1);
-    raster_occupancy(2);
+    raster_occupancy();
     for (int level = 1; level <= kMaxMsaaLog2; level++)
         ms_occupancy(level);
 }
@@ -2401,12 +2396,12 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
         default: k_raster_ms<32><<<blocks, threads, ms_smem(32), s>>>(a); break;
         }
     }
-    else if (a.tune.raster_variant == 2)
-        k_raster<6, false><<<raster_blocks(sms, a.tune), kRasterThreads, 0, s>>>(a);
-    else if (a.tune.raster_variant == 1)
-        k_raster<5, true><<<raster_blocks(sms, a.tune), kRasterThreads, 0, s>>>(a);
     else
-        k_raster<3, true><<<raster_blocks(sms, a.tune), kRasterThreads, 0, s>>>(a);
+    {
+        if (a.tune.raster_variant == 2)
+            a.tune.small_region = 0;
+        k_raster<<<raster_blocks(sms, a.tune), kRasterThreads, 0, s>>>(a);
+    }
     mark(5);
     return cudaGetLastError();
 }
