@@ -223,7 +223,7 @@ struct edxr_renderer
     DevBuf frames, frame_of_block, rtris, polys, clip_list, tile_count, tile_offset, tile_cursor, tile_zocc, bins, bin_tmp,
         big_list, counters,
         status;
-    DevBuf color, depth, tri_id, back8, diff_scratch, tri_first, items, keybuf, vrecs;
+    DevBuf color, depth, tri_id, back8, diff_scratch, tri_first, items, empty_tiles, keybuf, vrecs;
     // texture slots (edxr_set_textures): descriptors and the texel pool with mip chains
     DevBuf tex_desc, tex_texels;
     uint32_t num_textures = 0;
@@ -494,6 +494,7 @@ edxr_status launch_frames(edxr_renderer* r, uint32_t n, uint32_t width, uint32_t
     EDXR_CUDA(r->keybuf.ensure_zeroed(8 * samples * std::max<uint64_t>(pixels, 1), r->stream));
     const uint64_t icap = item_capacity(tiles, r->bin_capacity, (uint32_t)r->tuning.item_entries);
     EDXR_CUDA(r->items.ensure(sizeof(uint4) * icap));
+    EDXR_CUDA(r->empty_tiles.ensure(4 * std::max<uint64_t>(tiles, 1)));
     // a vertex stage when vertices are shared (on average by at least three
     // triangle corners) and their records stay in L2 for setup to gather
     // (up to 4 Mi vertices = 64 MiB of the 126 MiB): each vertex is then
@@ -543,6 +544,7 @@ edxr_status launch_frames(edxr_renderer* r, uint32_t n, uint32_t width, uint32_t
     a.tri_first = r->tri_first.as<uint32_t>();
     a.items = r->items.as<uint4>();
     a.item_capacity = icap;
+    a.empty_tiles = r->empty_tiles.as<uint32_t>();
     a.keybuf = r->keybuf.as<unsigned long long>();
     a.total_pixels = pixels;
     a.msaa_log2 = msaa_log2;
@@ -719,7 +721,7 @@ edxr_status edxr_destroy(edxr_renderer* r)
         cudaGraphExecDestroy(r->graph);
     DevBuf* bufs[] = { &r->frames, &r->frame_of_block, &r->rtris, &r->polys, &r->clip_list, &r->tile_count, &r->tile_offset,
                        &r->tile_cursor, &r->tile_zocc, &r->bins, &r->bin_tmp, &r->big_list, &r->counters, &r->status, &r->color,
-                       &r->depth, &r->tri_id, &r->back8, &r->diff_scratch, &r->tri_first, &r->items,
+                       &r->depth, &r->tri_id, &r->back8, &r->diff_scratch, &r->tri_first, &r->items, &r->empty_tiles,
                        &r->keybuf, &r->tex_desc, &r->tex_texels, &r->vrecs };
     for (DevBuf* b : bufs)
         b->release();

@@ -143,7 +143,7 @@ struct DeviceStatus
 struct Tuning
 {
     int small_region;     // bin entries whose pixel region is at most this are rasterized triangle-parallel
-    int raster_variant;   // 0/1: k_raster with the triangle-parallel path, 2: pixel-parallel only
+    int raster_variant;   // 0: a warp per raster item, 1: several where tiles are few, 2: as 1, pixel-parallel only
     int bin_blocks_per_sm;
     int raster_blocks_per_sm;  // 0 = as many as fit
     int item_entries;     // bin entries per raster work item; items of at least 3/4 of it are handed out first
@@ -185,12 +185,14 @@ struct PassArgs
     uint32_t big_capacity;
     uint32_t* counters;      // [0] fan-piece slots, [2] big tris, [3] raster work queue, [4] clip list,
                              // [6] heavy raster work items, [7] light ones, [8] scan block tickets,
+                             // [9] tiles with no bin entry,
                              // [11] surviving fan pieces, [kStripeBase + r * kStripeStride] stripe r of the
                              // unsorted bin list (kCounters words)
     unsigned long long* scan_status;  // per scan block (scan_blocks(total_tiles) words)
-    uint4* items;            // raster work items (tile | split flag, first entry, end entry, 0), one per
+    uint4* items;            // raster work items (tile | split flag, first entry, end entry, the bin's start), one per
                              // item_entries-entry slice: heavy ones from the front, light ones from the back
     uint64_t item_capacity;
+    uint32_t* empty_tiles;   // the tiles with no bin entry (counters[9] of them), total_tiles words
     unsigned long long* keybuf;  // per pixel: ~(smallest key) of split tiles, 0 between passes
     DeviceStatus* status;
     uint32_t* tri_first;     // per clipped input triangle: its first fan piece

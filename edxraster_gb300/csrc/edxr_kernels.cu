@@ -987,11 +987,12 @@ __global__ void __launch_bounds__(256, 4) k_bin_big(PassArgs a)
 // the ranges before them (scan_status: 0 not yet, kScanAggregate | sum of
 // the range, kScanPrefix | sum of everything up to the range's end).
 //
-// The same pass lists the raster work items: one per tile (an empty tile's
-// item writes its background) plus one per further tune.item_entries entries.
-// Items of at least 3/4 of that are listed from the front of the
-// item array, the lighter ones from its back, and the queue hands out the
-// front list first: the heavy work starts early instead of forming the tail.
+// The same pass lists the raster work items: one per tune.item_entries
+// entries of a tile.  Items of at least 3/4 of that are listed from the front
+// of the item array, the lighter ones from its back, and the queue hands out
+// the front list first: the heavy work starts early instead of forming the
+// tail.  Tiles without an entry, which only need their background, have a
+// list of their own.
 __device__ __forceinline__ uint32_t padded(uint32_t c) { return (c + 3u) & ~3u; }
 
 constexpr unsigned long long kScanAggregate = 1ull << 32;
@@ -1102,7 +1103,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
     // entries per work item; items of at least 3/4 of that are heavy
     const uint32_t E = (uint32_t)a.tune.item_entries, heavy_min = E - E / 4;
     uint32_t run = prefix + incl - sum;
-    uint32_t nheavy = 0, nlight = 0;
+    uint32_t nheavy = 0, nlight = 0, nempty = 0;
     uint32_t start[kScanItems], n[kScanItems];
 #pragma unroll
     for (int k = 0; k < kScanItems; k++)
@@ -1117,54 +1118,67 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
             a.tile_count[i] = 0;  // from here on: the split tile's rastered entries
             if (dropped || (uint64_t)run + c > a.bin_capacity)
                 c = 0;
-            n[k] = max(1u, (c + E - 1) / E);
+            n[k] = (c + E - 1) / E;
             // only the last item of a tile can be light
-            const uint32_t light = (c - (n[k] - 1) * E) < heavy_min ? 1u : 0u;
+            const uint32_t light = c && (c - (n[k] - 1) * E) < heavy_min ? 1u : 0u;
             nlight += light;
             nheavy += n[k] - light;
+            nempty += c ? 0u : 1u;
             cnt[k] = c;
         }
         run += padded(cnt[k]);
     }
-    // one atomic per warp and list (heavy count in the low half, light
-    // count in the high half of one word: at most 32 * 4 * 2^8 and 128)
+    // one atomic per warp and list (light and empty counts, at most 128 each,
+    // share a word)
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t packed = nheavy | (nlight << 24);
-    uint32_t pincl = packed;
+    const uint32_t packed = nlight | (nempty << 16);
+    uint32_t hincl = nheavy, pincl = packed;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1)
     {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, pincl, o);
-        if (lane >= (uint32_t)o) pincl += t;
+        const uint32_t h = __shfl_up_sync(0xffffffffu, hincl, o), t = __shfl_up_sync(0xffffffffu, pincl, o);
+        if (lane >= (uint32_t)o)
+        {
+            hincl += h;
+            pincl += t;
+        }
     }
-    uint32_t hbase = 0, lbase = 0;
+    uint32_t hbase = 0, lbase = 0, ebase = 0;
     if (lane == 31)
     {
-        if (pincl & 0xFFFFFFu)
-            hbase = atomicAdd(&a.counters[6], pincl & 0xFFFFFFu);
-        if (pincl >> 24)
-            lbase = atomicAdd(&a.counters[7], pincl >> 24);
+        if (hincl)
+            hbase = atomicAdd(&a.counters[6], hincl);
+        if (pincl & 0xFFFFu)
+            lbase = atomicAdd(&a.counters[7], pincl & 0xFFFFu);
+        if (pincl >> 16)
+            ebase = atomicAdd(&a.counters[9], pincl >> 16);
     }
     const uint32_t pexcl = pincl - packed;
-    hbase = __shfl_sync(0xffffffffu, hbase, 31) + (pexcl & 0xFFFFFFu);
-    lbase = __shfl_sync(0xffffffffu, lbase, 31) + (pexcl >> 24);
+    hbase = __shfl_sync(0xffffffffu, hbase, 31) + hincl - nheavy;
+    lbase = __shfl_sync(0xffffffffu, lbase, 31) + (pexcl & 0xFFFFu);
+    ebase = __shfl_sync(0xffffffffu, ebase, 31) + (pexcl >> 16);
 #pragma unroll
     for (int k = 0; k < kScanItems; k++)
     {
         const uint32_t i = base + k;
         if (i >= a.total_tiles)
             continue;
+        if (!cnt[k])
+        {
+            a.empty_tiles[ebase++] = i;
+            continue;
+        }
         const bool light = (cnt[k] - (n[k] - 1) * E) < heavy_min;
         const uint32_t heavy = n[k] - (light ? 1u : 0u);
         const uint32_t end = start[k] + cnt[k];
         const uint32_t tag = i | (n[k] > 1 ? kSplitTile : 0u);
         for (uint32_t j = 0; j < heavy; j++, hbase++)
             if (hbase < a.item_capacity)
-                a.items[hbase] = make_uint4(tag, start[k] + j * E, min(end, start[k] + (j + 1) * E), 0u);
+                a.items[hbase] = make_uint4(tag, start[k] + j * E, min(end, start[k] + (j + 1) * E), start[k]);
         if (light)
         {
             if (lbase < a.item_capacity)
-                a.items[a.item_capacity - 1 - lbase] = make_uint4(tag, start[k] + (n[k] - 1) * E, end, 0u);
+                a.items[a.item_capacity - 1 - lbase] = make_uint4(tag, start[k] + (n[k] - 1) * E, end, start[k]);
             lbase++;
         }
     }
@@ -1482,14 +1496,13 @@ static __device__ __forceinline__ void write_pixel_fast(const PixelOut a, const 
 // A tile shaded by the FP64 or the textured shader: out of line, pixel by
 // pixel, so that the common shaders' loop keeps its registers.
 static __device__ __noinline__ void shade_tile_slow(const PixelOut out, const FrameDesc& f,
-                                                    const unsigned long long* key, int tileX, int tileY, bool less,
-                                                    uint32_t nr, const uint32_t* tri_first, uint32_t total_tris)
+                                                    const unsigned long long* key, int first, int step, int tileX,
+                                                    int tileY, bool less, uint32_t nr, const uint32_t* tri_first,
+                                                    uint32_t total_tris)
 {
-    const uint32_t lane = threadIdx.x & 31;
 #pragma unroll 1
-    for (int k = 0; k < 8; k++)
+    for (int p = first; p < 256; p += step)
     {
-        const int p = (int)lane + 32 * k;
         const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
         if (px >= f.width || py >= f.height)
             continue;
@@ -1509,16 +1522,86 @@ static __device__ __noinline__ void shade_tile_slow(const PixelOut out, const Fr
     }
 }
 
+
+// Key of a covered fragment from its two unbiased edge values; a NaN depth,
+// which never passes, gives ~0.
+__device__ __forceinline__ unsigned long long depth_key64(int l1, int l2, const StagedTri& s, uint32_t rank)
+{
+    const float L0 = fmul(__int2float_rn(l1), s.invDet);
+    const float L1 = fmul(__int2float_rn(l2), s.invDet);
+    const float L2 = fsub(fsub(1.0f, L0), L1);
+    const float d = fadd(fadd(fmul(L0, s.z0), fmul(L1, s.z1)), fmul(L2, s.z2));
+    return d == d ? ((unsigned long long)depth_key(d) << 32) | rank : ~0ull;
+}
+
+// The background of a tile, written by `threads` threads.
+static __device__ __forceinline__ void clear_tile(const PassArgs& a, uint32_t tile, int thread, int threads)
+{
+    const uint32_t fi = a.tiles_per_frame ? tile / a.tiles_per_frame
+                                          : find_frame(a.frames, a.num_frames, tile,
+                                                       [](const FrameDesc& f) { return f.tile_base; });
+    const FrameDesc& f = a.frames[fi];
+    const uint32_t lt = tile - f.tile_base;
+    const int tileX = (int)(lt % (uint32_t)f.tdx), tileY = (int)(lt / (uint32_t)f.tdx);
+    const int w = f.width, h = f.height;
+    const uint64_t base = f.pix_base;
+    for (int p = thread; p < 256; p += threads)
+    {
+        const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
+        if (px < w && py < h)
+        {
+            const uint64_t pix = base + (uint64_t)py * (uint32_t)w + (uint32_t)px;
+            a.color[pix] = make_float4(0.f, 0.f, 0.f, 0.f);
+            a.depth[pix] = 1.0f;
+            a.tri_id[pix] = kNoTriangle;
+        }
+    }
+}
+
+// Barrier of the Group warps that share an item: the warp's own lanes
+// (Group 1), the whole block (Group 8), or a named barrier per group.
+template <int Group>
+__device__ __forceinline__ void group_sync(int group)
+{
+    if (Group == 1)
+        __syncwarp();
+    else if (Group == kRasterWarps)
+        __syncthreads();
+    else
+    {
+        __syncwarp();
+        asm volatile("bar.sync %0, %1;\n" ::"r"(group + 1), "r"(Group * 32) : "memory");
+    }
+}
+
+// Merges key k into a shared key: other warps of the group may write the same
+// one (Group > 1), or only this lane does.
+template <int Group>
+__device__ __forceinline__ void lower_key(unsigned long long* slot, unsigned long long k)
+{
+    if (Group == 1)
+        *slot = k;
+    else
+        atomicMin(slot, k);
+}
+
+// Group warps share an item (1: a warp per item; 2, 4 or 8 where the frame
+// has too few tiles to give every warp one, see raster_group).
 // 3 blocks per SM: the 80 registers a thread hold the shading without spills.
 // At 5 blocks (48 registers, 156 bytes spilled) the raster stage took 119
 // instead of 100 us on the terrain (2,097,152 triangles, 1920x1080), 235
 // instead of 217 on the binning stress (3840x2160), 67 instead of 55 on a
 // 301x301-quad terrain at 1366x769; at 4 blocks 109, 219 and 61; at 2 blocks
 // (124 registers) 111, 250 and 53.
+template <int Group>
 __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
 {
-    __shared__ unsigned long long s_key[kRasterWarps][256];
+    constexpr int kGroups = kRasterWarps / Group;   // groups of a block
+    constexpr int kThreads = 32 * Group;            // threads of a group
+    constexpr int kPixels = 256 / kThreads;         // pixels of the tile per thread
+    __shared__ unsigned long long s_key[kGroups][256];
     __shared__ StagedSlot s_tri[kRasterWarps][32];
+    __shared__ uint32_t s_next[kGroups], s_done[kGroups];
     if (*(volatile uint32_t*)&a.status->error)
         return;  // the pass failed (see k_bin_move); every thread of the block leaves
     // ceil(65536 / w): ((p * s_recip[w]) >> 16) == p / w for 0 <= p < 256 and
@@ -1528,7 +1611,10 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
         s_recip[threadIdx.x] = (65536u + threadIdx.x - 1u) / threadIdx.x;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long* key = s_key[warp];
+    const int group = (int)warp / Group;
+    const uint32_t gwarp = warp % Group;             // warp within the group
+    const int gthread = (int)(threadIdx.x % kThreads);
+    unsigned long long* key = s_key[group];
     StagedSlot* staged = s_tri[warp];
     // raster-triangle slots in use: one per input triangle, then the fan pieces
     const uint32_t nr = (uint32_t)min((uint64_t)a.total_tris + *(volatile uint32_t*)&a.counters[0],
@@ -1536,12 +1622,45 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
     const uint32_t nheavy = *(volatile uint32_t*)&a.counters[6];
     const uint32_t nitems = (uint32_t)min((uint64_t)nheavy + *(volatile uint32_t*)&a.counters[7], a.item_capacity);
     const int small_region = min(a.tune.small_region, 64);
+    const uint32_t before = (1u << lane) - 1u;  // lanes before this one
     const PixelOut out = { a.rtris, a.polys, a.color, a.depth, a.tri_id };
-    // each warp's first item is its own (the heaviest ones, no claim), the
-    // rest are claimed one at a time
-    for (uint32_t q = blockIdx.x * kRasterWarps + warp; q < nitems; q = claim_item(a, gridDim.x * kRasterWarps))
+    // The work: the items, then the tiles without an entry, a few at a time.
+    // Each group's first piece is its own (the heaviest items, no claim), the
+    // rest are claimed one at a time; nothing is claimed when every piece is
+    // some group's first (a claim on the one counter by every warp of the
+    // grid takes 3 to 6 us).  The empty tiles at the end fill the tail.  Where
+    // the items outnumber the groups, each item writes `share` of the empty
+    // tiles first, so that the background's stores overlap other warps'
+    // rasterization: 256 views at 512x512 768 -> 728 us.
+    const uint32_t nempty = *(volatile uint32_t*)&a.counters[9], ngroups = gridDim.x * kGroups;
+    const uint32_t share = nitems >= 2u * ngroups ? min(nempty / nitems, 4u) : 0u;
+    const uint32_t shared_tiles = share * nitems;
+    const uint32_t bulk = min(8u, max(1u, (nempty - shared_tiles) / ngroups));
+    const uint32_t nwork = nitems + (nempty - shared_tiles + bulk - 1) / bulk;
+    auto next_item = [&]() -> uint32_t {
+        if (ngroups >= nwork)
+            return nwork;
+        if (Group == 1)
+            return claim_item(a, ngroups);
+        if (gthread == 0)
+            s_next[group] = ngroups + atomicAdd(&a.counters[3], 1u);
+        group_sync<Group>(group);
+        return s_next[group];
+    };
+    for (uint32_t q = blockIdx.x * kGroups + group; q < nwork; q = next_item())
     {
+        if (q >= nitems)
+        {
+            const uint32_t i0 = shared_tiles + (q - nitems) * bulk, i1 = min(nempty, i0 + bulk);
+            for (uint32_t i = i0; i < i1; i++)
+                clear_tile(a, a.empty_tiles[i], gthread, kThreads);
+            if (Group > 1)
+                group_sync<Group>(group);
+            continue;
+        }
         const uint4 item = a.items[q < nheavy ? q : (uint32_t)(a.item_capacity - 1 - (q - nheavy))];
+        for (uint32_t i = 0; i < share; i++)
+            clear_tile(a, a.empty_tiles[q * share + i], gthread, kThreads);
         const uint32_t tile = item.x & ~kSplitTile;
         const uint32_t fi = a.tiles_per_frame ? tile / a.tiles_per_frame
                                               : find_frame(a.frames, a.num_frames, tile,
@@ -1555,68 +1674,64 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
         // the item's range within the entries its bin kept (the scatter drops
         // entries hidden behind the tile's occluder)
         uint32_t e0 = item.y, e1 = item.z, kept = 0;
+        const uint32_t c0 = e0 + 32 * gwarp;
+        uint32_t next = c0 + lane < e1 ? a.bins[c0 + lane] : 0u;
         if (e0 != e1)
         {
-            const uint32_t bin0 = a.tile_offset[tile];
+            const uint32_t bin0 = item.w;
             kept = a.tile_cursor[tile];
             e1 = min(e1, bin0 + kept);
             e0 = min(e0, e1);
             if (split && e0 == e1)
             {
                 if (item.y != bin0 || kept != 0)
-                    continue;  // the tile's kept entries are in its other items
+                {
+                    // the tile's kept entries are in its other items
+                    if (Group > 1)
+                        group_sync<Group>(group);
+                    continue;
+                }
                 split = false;  // it kept none: its first item writes the background
             }
         }
         if (e0 == e1 && !split)
         {
-            // a tile with no bin entry: its background, with no key
-            for (int k = 0; k < 8; k++)
-            {
-                const int p = (int)lane + 32 * k;
-                const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
-                if (px < f.width && py < f.height)
-                {
-                    const uint64_t pix = f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px;
-                    a.color[pix] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    a.depth[pix] = 1.0f;
-                    a.tri_id[pix] = kNoTriangle;
-                }
-            }
+            // every entry was hidden behind the clear depth: the background, with no key
+            clear_tile(a, tile, gthread, kThreads);
+            if (Group > 1)
+                group_sync<Group>(group);
             continue;
         }
 
         // clear depth 1.0 with no triangle: rank term ~0 (LEQUAL) or 0 (LESS)
         const unsigned long long clear = ((unsigned long long)0xBF800000u << 32) | (less ? 0u : 0xFFFFFFFFu);
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-            key[lane + 32 * k] = clear;
-        __syncwarp();
+        for (int k = 0; k < kPixels; k++)
+            key[gthread + kThreads * k] = clear;
+        group_sync<Group>(group);
         // depth bound of the tile: the nearest triangle that covers it whole,
         // then the largest depth key of its pixels so far
         const uint32_t tzocc = min(0xBF800000u, a.tile_zocc[tile]);
         uint32_t tzmax = tzocc;
 
         // each chunk's bin entries load while the previous chunk is rasterized
-        uint32_t next = e0 + lane < e1 ? a.bins[e0 + lane] : 0u;
-        for (uint32_t c = e0; c < e1; c += 32)
+        for (uint32_t c = c0; c < e1; c += kThreads)
         {
             const uint32_t m = min(32u, e1 - c);
             const uint32_t entry = next;
-            if (c + 32 + lane < e1)
-                next = a.bins[c + 32 + lane];
+            if (c + kThreads + lane < e1)
+                next = a.bins[c + kThreads + lane];
             int nsmall = 0;
             bool big = false;
+            StagedTri s;
             if (lane < m)
             {
-                StagedTri s;
                 uint32_t zk;
                 stage_tri(a, entry, nr, f.tri_base << 4, tileX, tileY, s, zk);
                 const uint32_t fl = s.flags;
                 const int rx0 = fl & 31, rx1 = (fl >> 5) & 31, ry0 = (fl >> 10) & 31, ry1 = (fl >> 15) & 31;
                 if (zk <= tzmax && rx0 <= rx1 && ry0 <= ry1)
                 {
-                    staged[lane].s = s;
                     const int area = (rx1 - rx0 + 1) * (ry1 - ry0 + 1);
                     if (!(fl & (1u << 20)) && area <= small_region)
                         nsmall = area;
@@ -1624,9 +1739,19 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                         big = true;
                 }
             }
+            // staged: the small entries, then the others
+            const uint32_t smalls = __ballot_sync(0xffffffffu, nsmall > 0), bigs = __ballot_sync(0xffffffffu, big);
+            const int nsm = __popc(smalls), nst = nsm + __popc(bigs);
+            if (nsmall > 0)
+                staged[__popc(smalls & before)].s = s;
+            else if (big)
+                staged[nsm + __popc(bigs & before)].s = s;
             // Small entries: their (entry, pixel) pairs are numbered across
             // the warp and taken 32 at a time, so lanes do not idle while
-            // one lane walks a larger region.
+            // one lane walks a larger region.  A lane finds its pair's entry
+            // from the entries that begin in the 32 pairs at hand, a lane mask
+            // (one warp-wide OR instead of five dependent shuffles of a
+            // search: terrain 102 -> 98 us).
             int incl = nsmall;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1)
@@ -1636,24 +1761,23 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
             }
             const int pairs = __shfl_sync(0xffffffffu, incl, 31);
             __syncwarp();
+            int started = -1, carry = 0;  // the last entry begun so far, and its pairs already taken
             for (int base = 0; base < pairs; base += 32)
             {
-                const int p = base + (int)lane;
-                // owner: the first lane whose inclusive count exceeds p
-                int j = 0;
-#pragma unroll
-                for (int st = 16; st >= 1; st >>= 1)
-                {
-                    const int v = __shfl_sync(0xffffffffu, incl, j + st - 1);
-                    if (v <= p) j += st;
-                }
-                const int first = __shfl_sync(0xffffffffu, incl - nsmall, j);
-                if (p < pairs)
+                // the entries that begin in this window, as a lane mask
+                const uint32_t begin = (uint32_t)(incl - nsmall - base);
+                const uint32_t heads = __reduce_or_sync(0xffffffffu, nsmall > 0 && begin < 32u ? 1u << begin : 0u);
+                const uint32_t upto = heads & (before | (1u << lane));
+                const int j = started + __popc(upto);
+                const int local = upto ? (int)lane - (31 - __clz(upto)) : carry + (int)lane;
+                started += __popc(heads);
+                carry = heads ? 32 - (31 - __clz(heads)) : carry + 32;
+                if (base + (int)lane < pairs)
                 {
                     const StagedTri s = staged[j].s;
                     const uint32_t fl = s.flags;
                     const int rx0 = fl & 31, rx1 = (fl >> 5) & 31, ry0 = (fl >> 10) & 31;
-                    const int rw = rx1 - rx0 + 1, local = p - first;
+                    const int rw = rx1 - rx0 + 1;
                     const int dy = (int)(((uint32_t)local * s_recip[rw]) >> 16);
                     const int x = rx0 + local - dy * rw, y = ry0 + dy;
                     uint64_t k;
@@ -1664,17 +1788,16 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                         atomicMin(&key[y * 16 + x], (unsigned long long)k);
                 }
             }
-            // Other entries: the whole warp over each region in turn.
-            uint32_t todo = __ballot_sync(0xffffffffu, big);
             __syncwarp();
-            while (todo)
+            // Other entries: the whole warp over each region in turn, in
+            // blocks of 16, 8 or 4 columns and two rows of blocks at a time.
+            for (int j = nsm; j < nst; j++)
             {
-                const int j = __ffs(todo) - 1;
-                todo &= todo - 1u;
                 const StagedTri s = staged[j].s;
                 const uint32_t fl = s.flags;
                 const int rx0 = fl & 31, rx1 = (fl >> 5) & 31, ry0 = (fl >> 10) & 31, ry1 = (fl >> 15) & 31;
-                const int rw = rx1 - rx0 + 1, area = rw * (ry1 - ry0 + 1);
+                const int rw = rx1 - rx0 + 1;
+                const int area = rw * (ry1 - ry0 + 1);
                 const uint32_t inv = s_recip[rw];
                 // each pixel of the region belongs to one lane for this entry
                 for (int p = (int)lane; p < area; p += 32)
@@ -1685,12 +1808,14 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                     const bool hit = fragment_key(s, x, y, less, k);
                     const unsigned long long cur = key[y * 16 + x];
                     if (hit && k < cur)
-                        key[y * 16 + x] = k;
+                        lower_key<Group>(&key[y * 16 + x], k);
                 }
                 __syncwarp();
             }
-            if (c + 32 < e1)
+            if (c + kThreads < e1)
             {
+                // (keys only fall, so a bound from keys that other warps are
+                // still lowering is a valid, larger one)
                 uint32_t mz = 0;
 #pragma unroll
                 for (int k = 0; k < 8; k++)
@@ -1698,6 +1823,8 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                 tzmax = min(tzocc, __reduce_max_sync(0xffffffffu, mz));
             }
         }
+        if (Group > 1)
+            group_sync<Group>(group);
 
         // A tile split into several items merges its keys in the key buffer;
         // the item that finishes last (the one whose entries bring the tile's
@@ -1707,30 +1834,40 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
         if (split)
         {
 #pragma unroll
-            for (int k = 0; k < 8; k++)
+            for (int k = 0; k < kPixels; k++)
             {
-                const int p = (int)lane + 32 * k;
+                const int p = gthread + kThreads * k;
                 const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
                 const unsigned long long kk = key[p];
                 if (px < f.width && py < f.height && kk < clear)
                     atomicMax(&a.keybuf[f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px], ~kk);
             }
-            // The count is one acquire-release atomic: the lanes' merges
-            // happen before it (warp barrier, then lane 0's release), and
-            // the item that completes the tile acquires every other item's
-            // merges before it reads them back.
-            __syncwarp();
-            uint32_t done = 0;
-            if (lane == 0)
-                done = atomic_add_acq_rel(&a.tile_count[tile], e1 - e0) + (e1 - e0);
-            shade = __shfl_sync(0xffffffffu, done, 0) == kept;
-            __syncwarp();  // lane 0's acquire, then every lane's reads
+            // The count is one acquire-release atomic: the group's merges
+            // happen before it (barrier, then its first thread's release),
+            // and the item that completes the tile acquires every other
+            // item's merges before it reads them back.
+            group_sync<Group>(group);
+            if (Group == 1)
+            {
+                uint32_t done = 0;
+                if (lane == 0)
+                    done = atomic_add_acq_rel(&a.tile_count[tile], e1 - e0) + (e1 - e0);
+                shade = __shfl_sync(0xffffffffu, done, 0) == kept;
+                __syncwarp();  // lane 0's acquire, then every lane's reads
+            }
+            else
+            {
+                if (gthread == 0)
+                    s_done[group] = atomic_add_acq_rel(&a.tile_count[tile], e1 - e0) + (e1 - e0);
+                group_sync<Group>(group);
+                shade = s_done[group] == kept;
+            }
             if (shade)
             {
 #pragma unroll
-                for (int k = 0; k < 8; k++)
+                for (int k = 0; k < kPixels; k++)
                 {
-                    const int p = (int)lane + 32 * k;
+                    const int p = gthread + kThreads * k;
                     const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
                     if (px < f.width && py < f.height)
                     {
@@ -1743,13 +1880,13 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
             }
         }
         if (shade && (f.ps_kind == 1 || f.ps_kind == 4))
-            shade_tile_slow(out, f, key, tileX, tileY, less, nr, a.tri_first, a.total_tris);
+            shade_tile_slow(out, f, key, gthread, kThreads, tileX, tileY, less, nr, a.tri_first, a.total_tris);
         else if (shade)
         {
 #pragma unroll 1
-            for (int k = 0; k < 8; k++)
+            for (int k = 0; k < kPixels; k++)
             {
-                const int p = (int)lane + 32 * k;
+                const int p = gthread + kThreads * k;
                 const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
                 const uint32_t low = (uint32_t)key[p];
                 const uint32_t ri = raster_triangle_of(a, less ? low : ~low, nr);
@@ -1757,7 +1894,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                     write_pixel_fast(out, f, ri, f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px, px, py);
             }
         }
-        __syncwarp();
+        group_sync<Group>(group);
     }
 }
 
@@ -1949,6 +2086,34 @@ static __device__ __noinline__ void shade_tile_ms_slow(const PassArgs& a, const 
     }
 }
 
+// The background of a tile with S samples, written by `threads` threads.
+template <int S>
+static __device__ __forceinline__ void clear_tile_ms(const PassArgs& a, uint32_t tile, int thread, int threads)
+{
+    const uint32_t fi = a.tiles_per_frame ? tile / a.tiles_per_frame
+                                          : find_frame(a.frames, a.num_frames, tile,
+                                                       [](const FrameDesc& f) { return f.tile_base; });
+    const FrameDesc& f = a.frames[fi];
+    const uint32_t lt = tile - f.tile_base;
+    const int tileX = (int)(lt % (uint32_t)f.tdx), tileY = (int)(lt / (uint32_t)f.tdx);
+    const int w = f.width, h = f.height;
+    const uint64_t base = f.pix_base, plane = a.total_pixels;
+    for (int p = thread; p < 256; p += threads)
+    {
+        const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
+        if (px >= w || py >= h)
+            continue;
+        const uint64_t pix = base + (uint64_t)py * (uint32_t)w + (uint32_t)px;
+        a.color[pix] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < S; s++)
+        {
+            a.depth[s * plane + pix] = 1.0f;
+            a.tri_id[s * plane + pix] = kNoTriangle;
+        }
+    }
+}
+
 // Raster with S samples per pixel: persistent blocks on the same work items as
 // k_raster.  A block's W warps share one tile and its keys [sample][pixel] in
 // dynamic shared memory: with a tile per warp the keys (2 KiB per sample) left
@@ -1978,7 +2143,6 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
 {
     constexpr int W = ms_warps(S);
     constexpr int kThreads = 32 * W;
-    constexpr int kPixels = 256 / kThreads;
     extern __shared__ unsigned long long ms_shared[];
     __shared__ uint32_t s_next, s_done, s_bound[W];
     if (*(volatile uint32_t*)&a.status->error)
@@ -1990,6 +2154,7 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
         s_recip[threadIdx.x] = (65536u + threadIdx.x - 1u) / threadIdx.x;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t before = (1u << lane) - 1u;  // lanes before this one
     unsigned long long* key = ms_shared;
     unsigned char* mine = reinterpret_cast<unsigned char*>(ms_shared + 256 * S) + warp * kMsWarpBytes;
     StagedMs* staged = reinterpret_cast<StagedMs*>(mine);
@@ -2000,7 +2165,13 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
     const uint32_t nheavy = *(volatile uint32_t*)&a.counters[6];
     const uint32_t nitems = (uint32_t)min((uint64_t)nheavy + *(volatile uint32_t*)&a.counters[7], a.item_capacity);
     const uint64_t plane = a.total_pixels;
+    const uint32_t nempty = *(volatile uint32_t*)&a.counters[9];
+    const uint32_t bulk = min(8u, max(1u, nempty / gridDim.x));
+    const uint32_t nwork = nitems + (nempty + bulk - 1) / bulk;
+    // the items, then the tiles without an entry, as in k_raster
     auto next_item = [&]() -> uint32_t {
+        if (gridDim.x >= nwork)
+            return nwork;
         if (threadIdx.x == 0)
             s_next = gridDim.x + atomicAdd(&a.counters[3], 1u);
         __syncthreads();
@@ -2008,8 +2179,16 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
     };
     // each block's first item is its own (the heaviest ones, no claim), the
     // rest are claimed one at a time
-    for (uint32_t q = blockIdx.x; q < nitems; q = next_item())
+    for (uint32_t q = blockIdx.x; q < nwork; q = next_item())
     {
+        if (q >= nitems)
+        {
+            const uint32_t i0 = (q - nitems) * bulk, i1 = min(nempty, i0 + bulk);
+            for (uint32_t i = i0; i < i1; i++)
+                clear_tile_ms<S>(a, a.empty_tiles[i], (int)threadIdx.x, kThreads);
+            __syncthreads();
+            continue;
+        }
         const uint4 item = a.items[q < nheavy ? q : (uint32_t)(a.item_capacity - 1 - (q - nheavy))];
         const uint32_t tile = item.x & ~kSplitTile;
         const uint32_t fi = a.tiles_per_frame ? tile / a.tiles_per_frame
@@ -2026,7 +2205,7 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
         uint32_t e0 = item.y, e1 = item.z, kept = 0;
         if (e0 != e1)
         {
-            const uint32_t bin0 = a.tile_offset[tile];
+            const uint32_t bin0 = item.w;
             kept = a.tile_cursor[tile];
             e1 = min(e1, bin0 + kept);
             e0 = min(e0, e1);
@@ -2042,23 +2221,8 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
         }
         if (e0 == e1 && !split)
         {
-            // a tile with no bin entry: its background, with no key
-            for (int k = 0; k < kPixels; k++)
-            {
-                const int p = (int)threadIdx.x + kThreads * k;
-                const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
-                if (px < f.width && py < f.height)
-                {
-                    const uint64_t pix = f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px;
-                    a.color[pix] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (int s = 0; s < S; s++)
-                    {
-                        a.depth[s * plane + pix] = 1.0f;
-                        a.tri_id[s * plane + pix] = kNoTriangle;
-                    }
-                }
-            }
+            // every entry was hidden behind the clear depth: the background, with no key
+            clear_tile_ms<S>(a, tile, (int)threadIdx.x, kThreads);
             __syncthreads();
             continue;
         }
@@ -2112,35 +2276,37 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
         {
             const uint32_t m = min(32u, e1 - c);
             int area = 0;
+            StagedTri st;
+            int G[3];
+            bool wfree = false;
             if (lane < m)
             {
-                StagedTri st;
                 uint32_t zk;
-                int G[3];
-                bool wfree = false;
                 stage_tri<true>(a, a.bins[c + lane], nr, f.tri_base << 4, tileX, tileY, st, zk, G, &wfree);
                 const uint32_t fl = st.flags;
                 const int rx0 = fl & 31, rx1 = (fl >> 5) & 31, ry0 = (fl >> 10) & 31, ry1 = (fl >> 15) & 31;
                 if (zk <= tzmax && rx0 <= rx1 && ry0 <= ry1)
-                {
-                    StagedMs& t = staged[lane];
-                    t.A0 = st.A0; t.D0 = st.D0; t.A1 = st.A1; t.D1 = st.D1; t.A2 = st.A2; t.D2 = st.D2;
-                    t.K0 = st.K0; t.K1 = st.K1; t.K2 = st.K2;
-                    t.G0 = G[0]; t.G1 = G[1]; t.G2 = G[2];
-                    // the largest o * G over the offsets [-8, 7] of any sample table
-                    t.Q0 = wadd(st.K0, G[0] > 0 ? wmul(7, G[0]) : wmul(-8, G[0]));
-                    t.Q1 = wadd(st.K1, G[1] > 0 ? wmul(7, G[1]) : wmul(-8, G[1]));
-                    t.Q2 = wadd(st.K2, G[2] > 0 ? wmul(7, G[2]) : wmul(-8, G[2]));
-                    t.flags = fl | ((fl & (1u << 20)) || !wfree ? (1u << 23) : 0u);
-                    t.rank = st.rank;
-                    t.invDet = st.invDet; t.z0 = st.z0; t.z1 = st.z1; t.z2 = st.z2;
                     area = (rx1 - rx0 + 1) * (ry1 - ry0 + 1);
-                }
+            }
+            const uint32_t live = __ballot_sync(0xffffffffu, area > 0);
+            if (area > 0)
+            {
+                StagedMs& t = staged[__popc(live & before)];
+                t.A0 = st.A0; t.D0 = st.D0; t.A1 = st.A1; t.D1 = st.D1; t.A2 = st.A2; t.D2 = st.D2;
+                t.K0 = st.K0; t.K1 = st.K1; t.K2 = st.K2;
+                t.G0 = G[0]; t.G1 = G[1]; t.G2 = G[2];
+                // the largest o * G over the offsets [-8, 7] of any sample table
+                t.Q0 = wadd(st.K0, G[0] > 0 ? wmul(7, G[0]) : wmul(-8, G[0]));
+                t.Q1 = wadd(st.K1, G[1] > 0 ? wmul(7, G[1]) : wmul(-8, G[1]));
+                t.Q2 = wadd(st.K2, G[2] > 0 ? wmul(7, G[2]) : wmul(-8, G[2]));
+                t.flags = st.flags | ((st.flags & (1u << 20)) || !wfree ? (1u << 23) : 0u);
+                t.rank = st.rank;
+                t.invDet = st.invDet; t.z0 = st.z0; t.z1 = st.z1; t.z2 = st.z2;
             }
             // (entry, pixel) pairs numbered across the warp and taken 32 at a
-            // time, so lanes do not idle on entries of a few pixels; pixels
-            // with a sample that may be covered are queued and, 32 at a time
-            // again, their S samples tested
+            // time (as in k_raster), so lanes do not idle on entries of a few
+            // pixels; pixels with a sample that may be covered are queued
+            // and, 32 at a time again, their S samples tested
             int incl = area;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1)
@@ -2150,27 +2316,24 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
             }
             const int pairs = __shfl_sync(0xffffffffu, incl, 31);
             __syncwarp();
-            int queued = 0;
+            int queued = 0, started = -1, carry = 0;
             for (int base = 0; base < pairs; base += 32)
             {
-                const int p = base + (int)lane;
-                // owner: the first lane whose inclusive count exceeds p
-                int j = 0;
-#pragma unroll
-                for (int st = 16; st >= 1; st >>= 1)
-                {
-                    const int v = __shfl_sync(0xffffffffu, incl, j + st - 1);
-                    if (v <= p) j += st;
-                }
-                const int first = __shfl_sync(0xffffffffu, incl - area, j);
+                const uint32_t begin = (uint32_t)(incl - area - base);
+                const uint32_t heads = __reduce_or_sync(0xffffffffu, area > 0 && begin < 32u ? 1u << begin : 0u);
+                const uint32_t upto = heads & (before | (1u << lane));
+                const int j = started + __popc(upto);
+                const int local = upto ? (int)lane - (31 - __clz(upto)) : carry + (int)lane;
+                started += __popc(heads);
+                carry = heads ? 32 - (31 - __clz(heads)) : carry + 32;
                 bool keep = false;
                 uint32_t e = 0;
-                if (p < pairs)
+                if (base + (int)lane < pairs)
                 {
                     const StagedMs& st = staged[j];
                     const uint32_t fl = st.flags;
                     const int rx0 = fl & 31, rx1 = (fl >> 5) & 31, ry0 = (fl >> 10) & 31;
-                    const int rw = rx1 - rx0 + 1, local = p - first;
+                    const int rw = rx1 - rx0 + 1;
                     const int dy = (int)(((uint32_t)local * s_recip[rw]) >> 16);
                     const int x = rx0 + local - dy * rw, y = ry0 + dy;
                     e = ((uint32_t)j << 8) | (uint32_t)(y * 16 + x);
@@ -2178,7 +2341,7 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
                 }
                 const uint32_t kept_lanes = __ballot_sync(0xffffffffu, keep);
                 if (keep)
-                    queue[queued + __popc(kept_lanes & ((1u << lane) - 1u))] = (uint16_t)e;
+                    queue[queued + __popc(kept_lanes & before)] = (uint16_t)e;
                 queued += __popc(kept_lanes);
                 __syncwarp();
                 if (queued >= 32)
@@ -2281,26 +2444,50 @@ __global__ void k_back_buffer(const float4* color, uchar4* out, int width, int h
 
 // -------------------------------------------------------------------------
 
-// Resident blocks per SM of k_raster.
+// Resident blocks per SM of k_raster<Group>.
+template <int Group>
 static int raster_occupancy()
 {
     static int per_sm = 0;
     if (!per_sm)
     {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_raster, kRasterThreads, 0) != cudaSuccess || n < 1)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_raster<Group>, kRasterThreads, 0) != cudaSuccess || n < 1)
             n = 1;
         per_sm = n;
     }
     return per_sm;
 }
 
-static int raster_blocks(int sms, const Tuning& t)
+template <int Group>
+static void launch_raster(int sms, const PassArgs& a, cudaStream_t s)
 {
-    int per = raster_occupancy();
-    if (t.raster_blocks_per_sm > 0 && t.raster_blocks_per_sm < per)
-        per = t.raster_blocks_per_sm;
-    return sms * per;
+    int per = raster_occupancy<Group>();
+    if (a.tune.raster_blocks_per_sm > 0 && a.tune.raster_blocks_per_sm < per)
+        per = a.tune.raster_blocks_per_sm;
+    k_raster<Group><<<sms * per, kRasterThreads, 0, s>>>(a);
+}
+
+// Warps per raster item.  A warp alone takes 10 to 25 us for a tile (a chain
+// of dependent loads, then eight rounds of shading), so a frame with fewer
+// tiles than resident warps (24 per SM) leaves most of the chip idle for that
+// long; more warps per tile shorten it.  Against it stand the barriers and,
+// with more than one warp, a 64-bit shared atomic per pixel of a large region
+// instead of a store, so frames of few triangles per tile (large regions) and
+// frames with several tiles per warp keep one.  Raster stage, 1 / 2 / 4 / 8
+// warps, us: sphere (4,032 triangles) 320x180, 240 tiles, 27.6 / 20.1 / 18.4 /
+// 16.4; 128x128-quad terrain 640x400, 1,000 tiles, 42.3 / 33.8 / 32.4 / 30.4;
+// 200x200 quads 800x520, 1,650 tiles, 47.1 / 36.5 / 35.8 / 36.2; 256x256 quads
+// 1280x720, 3,600 tiles, textured, 76 / 67; 301x301 quads 1366x769, 4,214
+// tiles, 56 / 53; sphere 1280x720 (1.1 triangles per tile) 24.6 / 28.7;
+// 2,097,152-triangle terrain, 8,160 tiles, 96 / 99; binning stress, 32,400
+// tiles, 215 / 310.
+static int raster_group(const PassArgs& a, int sms)
+{
+    const uint64_t tiles = a.total_tiles, warps = 24ull * (uint64_t)sms;
+    if (a.tune.raster_variant == 0 || a.total_tris < 8 * tiles)
+        return 1;
+    return 8 * tiles <= warps + warps / 8 ? 8 : 2 * tiles <= warps ? 4 : tiles <= warps + warps / 4 ? 2 : 1;
 }
 
 // Resident blocks per SM of k_raster_ms with 2^level samples (the dynamic
@@ -2337,7 +2524,10 @@ static int ms_occupancy(int level)
 
 void prepare_kernels()
 {
-    raster_occupancy();
+    raster_occupancy<1>();
+    raster_occupancy<2>();
+    raster_occupancy<4>();
+    raster_occupancy<8>();
     for (int level = 1; level <= kMaxMsaaLog2; level++)
         ms_occupancy(level);
 }
@@ -2358,12 +2548,14 @@ Tuning default_tuning()
 cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* ev)
 {
     PassArgs a = pass;
+    const int sms = a.num_sms > 0 ? a.num_sms : 148;
     // With several samples a block of warps shares an item, so an item takes
     // more entries (twice, four times with 8 warps): 4 samples of the terrain
     // 309 -> 303 us, 16 samples 381 -> 317.
     if (a.msaa_log2 > 0)
         a.tune.item_entries = min(1024, a.tune.item_entries * (a.msaa_log2 <= 3 ? 2 : 4));
-    const int sms = a.num_sms > 0 ? a.num_sms : 148;
+    else
+        a.tune.item_entries = min(1024, a.tune.item_entries * raster_group(a, sms));
     const uint32_t nscan = scan_blocks(a.total_tiles);
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
@@ -2400,7 +2592,13 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
     {
         if (a.tune.raster_variant == 2)
             a.tune.small_region = 0;
-        k_raster<<<raster_blocks(sms, a.tune), kRasterThreads, 0, s>>>(a);
+        switch (raster_group(a, sms))
+        {
+        case 8: launch_raster<8>(sms, a, s); break;
+        case 4: launch_raster<4>(sms, a, s); break;
+        case 2: launch_raster<2>(sms, a, s); break;
+        default: launch_raster<1>(sms, a, s); break;
+        }
     }
     mark(5);
     return cudaGetLastError();

@@ -290,8 +290,9 @@ typedef struct edxr_tuning
 {
     int small_region;             /* bin entries whose pixel region in a 16x16 tile is at most this
                                      many pixels are rasterized one triangle per thread; 0 disables */
-    int raster_variant;           /* 0, 1: raster kernel with the triangle-parallel path;
-                                     2: pixel-parallel only (small_region ignored) */
+    int raster_variant;           /* 0: one warp per raster work item; 1: one, or several where the
+                                     frame has few tiles; 2: as 1, pixel-parallel only (small_region
+                                     ignored) */
     int bin_blocks_per_sm;        /* grid of the per-triangle binning kernels */
     int raster_blocks_per_sm;     /* persistent raster blocks per SM; 0 = the occupancy maximum */
     uint32_t bin_entries_per_triangle;  /* initial bin-buffer capacity per triangle (grows on overflow) */
