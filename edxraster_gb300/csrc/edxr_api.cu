@@ -223,7 +223,7 @@ struct edxr_renderer
     DevBuf frames, frame_of_block, rtris, polys, clip_list, tile_count, tile_offset, tile_cursor, tile_zocc, bins, bin_tmp,
         big_list, counters,
         status;
-    DevBuf color, depth, tri_id, back8, diff_scratch, tri_first, items, empty_tiles, keybuf, vrecs;
+    DevBuf color, depth, tri_id, back8, diff_scratch, diff_packed, tri_first, items, empty_tiles, keybuf, vrecs;
     // texture slots (edxr_set_textures): descriptors and the texel pool with mip chains
     DevBuf tex_desc, tex_texels;
     uint32_t num_textures = 0;
@@ -721,7 +721,7 @@ edxr_status edxr_destroy(edxr_renderer* r)
         cudaGraphExecDestroy(r->graph);
     DevBuf* bufs[] = { &r->frames, &r->frame_of_block, &r->rtris, &r->polys, &r->clip_list, &r->tile_count, &r->tile_offset,
                        &r->tile_cursor, &r->tile_zocc, &r->bins, &r->bin_tmp, &r->big_list, &r->counters, &r->status, &r->color,
-                       &r->depth, &r->tri_id, &r->back8, &r->diff_scratch, &r->tri_first, &r->items, &r->empty_tiles,
+                       &r->depth, &r->tri_id, &r->back8, &r->diff_scratch, &r->diff_packed, &r->tri_first, &r->items, &r->empty_tiles,
                        &r->keybuf, &r->tex_desc, &r->tex_texels, &r->vrecs };
     for (DevBuf* b : bufs)
         b->release();
@@ -1241,7 +1241,11 @@ edxr_status edxr_backward(edxr_renderer* r, const edxr_mesh* mesh, const edxr_sh
     edxr_status s = diff_mesh(r, mesh, params, &m);
     if (s != EDXR_OK)
         return s;
-    EDXR_CUDA(r->diff_scratch.ensure(8 * sizeof(double)));
+    const uint64_t total = (uint64_t)r->last_frames * r->out_width * r->out_height;
+    EDXR_CUDA(r->diff_scratch.ensure_zeroed(8 * sizeof(double), r->stream));
+    const bool packed = packed_gradients(total, m.nv) && (grads->albedo || grads->normals || grads->positions);
+    if (packed)
+        EDXR_CUDA(r->diff_packed.ensure_zeroed(sizeof(float) * kPackedFloats * (size_t)m.nv, r->stream));
     DiffGrads dg;
     dg.albedo = grads->albedo;
     dg.normals = grads->normals;
@@ -1250,7 +1254,7 @@ edxr_status edxr_backward(edxr_renderer* r, const edxr_mesh* mesh, const edxr_sh
     dg.ks = grads->ks;
     dg.shininess = grads->shininess;
     dg.scratch = r->diff_scratch.as<double>();
-    const uint64_t total = (uint64_t)r->last_frames * r->out_width * r->out_height;
+    dg.packed = packed ? r->diff_packed.as<float>() : nullptr;
     EDXR_CUDA(launch_backward(r->last, total, m, reinterpret_cast<const float4*>(grad_color), dg, r->stream));
     EDXR_CUDA(cudaEventRecord(r->done, r->stream));
     return EDXR_OK;

@@ -241,12 +241,18 @@ struct DiffMesh
     int override_shading;   // 1: use light/ks/shininess below for every frame
     float light[3], ks, shininess;
 };
+constexpr int kPackedFloats = 12;  // per vertex: albedo, normal and position gradient, 3 unused
 struct DiffGrads
 {
     float* albedo; float* normals; float* positions;  // nv*3 each, may be NULL
     float* light; float* ks; float* shininess;         // may be NULL
-    double* scratch;                                    // 5 doubles, zeroed by the launcher
+    double* scratch;                                    // 5 doubles, zero between calls
+    float* packed;                                      // NULL, or nv * kPackedFloats, zero between calls
 };
+// Are the per-vertex gradients summed in a packed array first?  Clearing and
+// adding it costs 132 bytes of traffic a vertex, the sums in place 18
+// reductions more a covered pixel.
+constexpr bool packed_gradients(uint64_t pixels, uint64_t vertices) { return vertices > 0 && 4 * vertices <= pixels; }
 cudaError_t launch_shade_visible(const PassArgs& a, uint64_t total_pixels, const DiffMesh& m, float4* out,
                                  cudaStream_t s);
 cudaError_t launch_backward(const PassArgs& a, uint64_t total_pixels, const DiffMesh& m, const float4* grad,
