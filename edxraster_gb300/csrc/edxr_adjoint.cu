@@ -26,7 +26,13 @@ namespace edxr {
 
 namespace {
 
-constexpr int kThreads = 256;
+// A warp takes kSpan or fewer consecutive pixels, lists the covered ones and
+// shades those 32 at a time: with a thread per pixel, rows that the mesh covers
+// in part left lanes and whole warps of a block idle (21 to 31 % of the warps
+// active on 64 views of a torus, 30 % of the pixels covered).
+constexpr int kWarps = 4;
+constexpr int kThreads = 32 * kWarps;
+constexpr int kSpan = 256;
 
 // Frame of flattened output pixel p: one division when the pass's frames
 // share one resolution (tiles_per_frame set: the batched pass), else a
@@ -259,24 +265,68 @@ __device__ __forceinline__ V3 shade_forward(const FrameDesc& f, const Shading& s
     return v3(t.diffuse + t.spec, t.diffuse + t.spec, t.diffuse + t.spec);
 }
 
-__global__ void __launch_bounds__(kThreads) k_shade_visible(PassArgs a, uint64_t total, DiffMesh m, float4* out)
+// The covered pixels of a warp's span, in order.
+struct Covered
 {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total)
-        return;
-    const FrameDesc& f = a.frames[frame_of_pixel(a, i)];
-    const uint64_t local = i - f.pix_base;
-    const int px = (int)(local % (uint32_t)f.width), py = (int)(local / (uint32_t)f.width);
-    const uint32_t tri = a.tri_id[i];
-    PixelState s;
-    if (tri == kNoTriangle || !pixel_forward(f, m, tri, px, py, s))
+    uint32_t tri[kSpan];
+    uint8_t at[kSpan];
+};
+
+// Lists the covered pixels among [base, base + 32 * rows) below `total`;
+// `empty(pixel)` is called for the others.  Every lane of the warp calls it.
+template <typename Empty>
+__device__ __forceinline__ int list_covered(const PassArgs& a, uint64_t base, int rows, uint64_t total, uint32_t nt,
+                                            Covered& list, Empty empty)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t tri[kSpan / 32];
+#pragma unroll
+    for (int k = 0; k < kSpan / 32; k++)
+        tri[k] = k < rows && base + 32 * k + lane < total ? __ldg(a.tri_id + base + 32 * k + lane) : kNoTriangle;
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < kSpan / 32; k++)
     {
-        out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        return;
+        const bool covered = tri[k] < nt;
+        const uint32_t lanes = __ballot_sync(0xffffffffu, covered);
+        if (covered)
+        {
+            const int slot = n + __popc(lanes & ((1u << lane) - 1u));
+            list.tri[slot] = tri[k];
+            list.at[slot] = (uint8_t)(32 * k + lane);
+        }
+        else if (k < rows && base + 32 * k + lane < total)
+            empty(base + 32 * k + lane);
+        n += __popc(lanes);
     }
-    ShadeTerms t;
-    const V3 c = shade_forward(f, shading_of(f, m), s, t);
-    out[i] = make_float4(c.x, c.y, c.z, 1.0f);
+    __syncwarp();
+    return n;
+}
+
+__global__ void __launch_bounds__(kThreads, 5) k_shade_visible(PassArgs a, uint64_t total, int rows, DiffMesh m,
+                                                            float4* out)
+{
+    __shared__ Covered s_list[kWarps];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t base = ((uint64_t)blockIdx.x * kWarps + warp) * (32u * (uint32_t)rows);
+    const int n = list_covered(a, base, rows, total, m.nt, s_list[warp],
+                               [&](uint64_t i) { out[i] = make_float4(0.f, 0.f, 0.f, 0.f); });
+    for (int b = (int)lane; b < n; b += 32)
+    {
+        const uint64_t i = base + s_list[warp].at[b];
+        const FrameDesc& f = a.frames[frame_of_pixel(a, i)];
+        const uint64_t local = i - f.pix_base;
+        const int px = (int)(local % (uint32_t)f.width), py = (int)(local / (uint32_t)f.width);
+        PixelState s;
+        float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (pixel_forward(f, m, s_list[warp].tri[b], px, py, s))
+        {
+            ShadeTerms t;
+            const V3 x = shade_forward(f, shading_of(f, m), s, t);
+            c = make_float4(x.x, x.y, x.z, 1.0f);
+        }
+        out[i] = c;
+    }
 }
 
 __device__ __forceinline__ void add3(float* g, uint32_t v, V3 d)
@@ -309,121 +359,131 @@ __device__ __forceinline__ void add_packed(float* sums, uint32_t v, V3 da, V3 dn
 // reductions a vertex (two of 16 bytes), and added to the caller's arrays by
 // k_finish; otherwise straight into the caller's arrays, nine 4-byte
 // reductions a vertex.  The reductions bounded the kernel: 50,000 triangles
-// in 64 views of 256x256, 1.3 M covered pixels, 51 M reduction sectors in L2.
+// in 64 views of 256x256, 1.3 M covered pixels, 51 M reduction sectors in L2,
+// 311 us; packed 236; with the covered pixels of a span listed first (and
+// one double reduction of the global sums per 1,024 pixels instead of 256)
+// 151, and k_shade_visible 118 -> 89.  4 blocks of 128 per SM (121 registers)
+// against 5 (96, 40 bytes spilled) measured 151 and 148 us, 6 157.
 template <bool Packed>
-__global__ void __launch_bounds__(kThreads) k_backward(PassArgs a, uint64_t total, DiffMesh m, const float4* grad,
-                                                       DiffGrads g)
+__global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t total, int rows, DiffMesh m,
+                                                       const float4* grad, DiffGrads g)
 {
-    __shared__ float red[5 * (kThreads / 32)];
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    V3 dl = v3(0.f, 0.f, 0.f);
-    float dks = 0.0f, dshin = 0.0f;
-    if (i < total)
+    __shared__ Covered s_list[kWarps];
+    __shared__ double red[kWarps][5];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t base = ((uint64_t)blockIdx.x * kWarps + warp) * (32u * (uint32_t)rows);
+    const int n = list_covered(a, base, rows, total, m.nt, s_list[warp], [](uint64_t) {});
+    double sums[5] = { 0.0, 0.0, 0.0, 0.0, 0.0 };  // of the warp, lane 0
+    for (int b0 = 0; b0 < n; b0 += 32)
     {
-        const FrameDesc& f = a.frames[frame_of_pixel(a, i)];
-        const uint64_t local = i - f.pix_base;
-        const int px = (int)(local % (uint32_t)f.width), py = (int)(local / (uint32_t)f.width);
-        const uint32_t tri = a.tri_id[i];
-        PixelState s;
-        if (tri != kNoTriangle && pixel_forward(f, m, tri, px, py, s))
+        V3 dl = v3(0.f, 0.f, 0.f);
+        float dks = 0.0f, dshin = 0.0f;
+        if (b0 + (int)lane < n)
         {
-            ShadeTerms t;
-            const Shading sh = shading_of(f, m);
-            shade_forward(f, sh, s, t);
-            const float4 gc = grad[i];
-            const V3 gcol = v3(gc.x, gc.y, gc.z);
-            // colour = (albedo ? A * diffuse : diffuse) + spec
-            const V3 dA = t.albedo ? t.diffuse * gcol : v3(0.f, 0.f, 0.f);
-            const float ddiff = t.albedo ? dot(gcol, s.A) : (gcol.x + gcol.y + gcol.z);
-            const float dspec = t.specular ? (gcol.x + gcol.y + gcol.z) : 0.0f;
-            V3 dNn = v3(0.f, 0.f, 0.f), dL = v3(0.f, 0.f, 0.f), dP = v3(0.f, 0.f, 0.f);
-            // diffuse = (max(nl, 0) + 0.2) * 3/pi
-            const float dnl = (t.nl > 0.0f) ? ddiff * 0.954929658551372f : 0.0f;
-            dL = dL + dnl * t.Nn;
-            dNn = dNn + dnl * t.L;
-            if (t.specular)
+            const uint64_t i = base + s_list[warp].at[b0 + lane];
+            const uint32_t tri = s_list[warp].tri[b0 + lane];
+            const FrameDesc& f = a.frames[frame_of_pixel(a, i)];
+            const uint64_t local = i - f.pix_base;
+            const int px = (int)(local % (uint32_t)f.width), py = (int)(local / (uint32_t)f.width);
+            PixelState s;
+            if (pixel_forward(f, m, tri, px, py, s))
             {
-                // spec = ks * nhc^s
-                dks = dspec * t.powv;
-                if (t.nhc > 0.0f)
-                    dshin = dspec * sh.ks * t.powv * logf(t.nhc);
-                float dnh = 0.0f;
-                if (!t.clamp || t.nh > 0.0f)
+                ShadeTerms t;
+                const Shading sh = shading_of(f, m);
+                shade_forward(f, sh, s, t);
+                const float4 gc = grad[i];
+                const V3 gcol = v3(gc.x, gc.y, gc.z);
+                // colour = (albedo ? A * diffuse : diffuse) + spec
+                const V3 dA = t.albedo ? t.diffuse * gcol : v3(0.f, 0.f, 0.f);
+                const float ddiff = t.albedo ? dot(gcol, s.A) : (gcol.x + gcol.y + gcol.z);
+                const float dspec = t.specular ? (gcol.x + gcol.y + gcol.z) : 0.0f;
+                V3 dNn = v3(0.f, 0.f, 0.f), dL = v3(0.f, 0.f, 0.f), dP = v3(0.f, 0.f, 0.f);
+                // diffuse = (max(nl, 0) + 0.2) * 3/pi
+                const float dnl = (t.nl > 0.0f) ? ddiff * 0.954929658551372f : 0.0f;
+                dL = dL + dnl * t.Nn;
+                dNn = dNn + dnl * t.L;
+                if (t.specular)
                 {
-                    // nhc^(s - 1) from nhc^s where that is far from underflow
-                    const float p1 = fabsf(t.powv) > 1e-30f ? t.powv / t.nhc : powf(t.nhc, sh.shininess - 1.0f);
-                    dnh = (sh.shininess == 0.0f) ? 0.0f : dspec * sh.ks * sh.shininess * p1;
+                    // spec = ks * nhc^s
+                    dks = dspec * t.powv;
+                    if (t.nhc > 0.0f)
+                        dshin = dspec * sh.ks * t.powv * logf(t.nhc);
+                    float dnh = 0.0f;
+                    if (!t.clamp || t.nh > 0.0f)
+                    {
+                        // nhc^(s - 1) from nhc^s where that is far from underflow
+                        const float p1 = fabsf(t.powv) > 1e-30f ? t.powv / t.nhc : powf(t.nhc, sh.shininess - 1.0f);
+                        dnh = (sh.shininess == 0.0f) ? 0.0f : dspec * sh.ks * sh.shininess * p1;
+                    }
+                    dNn = dNn + dnh * t.H;
+                    const V3 dH = dnh * t.Nn;
+                    const V3 dHr = normalize_grad(t.H, t.hlen, dH);  // H = normalize(L + E)
+                    dL = dL + dHr;
+                    const V3 dEr = normalize_grad(t.E, t.elen, dHr);  // E = normalize(eye - P)
+                    dP = dP - dEr;
                 }
-                dNn = dNn + dnh * t.H;
-                const V3 dH = dnh * t.Nn;
-                const V3 dHr = normalize_grad(t.H, t.hlen, dH);  // H = normalize(L + E)
-                dL = dL + dHr;
-                const V3 dEr = normalize_grad(t.E, t.elen, dHr);  // E = normalize(eye - P)
-                dP = dP - dEr;
-            }
-            const V3 dNraw = normalize_grad(t.Nn, t.nlen, dNn);
-            dl = normalize_grad(t.L, t.llen, dL);
-            // P, N, A = sum b_k (p_k, n_k, a_k)
-            float db[3];
-            for (int k = 0; k < 3; k++)
-                db[k] = dot(dP, s.p[k]) + dot(dNraw, s.n[k]) + dot(dA, s.a[k]);
-            // b = bt / S
-            const float bdb = s.b[0] * db[0] + s.b[1] * db[1] + s.b[2] * db[2];
-            float dbt[3];
-            for (int k = 0; k < 3; k++)
-                dbt[k] = (db[k] - bdb) / s.S;
-            // bt = a x c
-            float dac[3] = { 0.f, 0.f, 0.f }, dcc[3] = { 0.f, 0.f, 0.f };
-            dac[1] += dbt[0] * s.cc[2]; dcc[2] += dbt[0] * s.ac[1]; dac[2] -= dbt[0] * s.cc[1]; dcc[1] -= dbt[0] * s.ac[2];
-            dac[2] += dbt[1] * s.cc[0]; dcc[0] += dbt[1] * s.ac[2]; dac[0] -= dbt[1] * s.cc[2]; dcc[2] -= dbt[1] * s.ac[0];
-            dac[0] += dbt[2] * s.cc[1]; dcc[1] += dbt[2] * s.ac[0]; dac[1] -= dbt[2] * s.cc[0]; dcc[0] -= dbt[2] * s.ac[1];
-            // a_k = X_k - u W_k, c_k = Y_k - v W_k, (X, Y, W) = rows 0, 1, 3 of MVP (p, 1)
-            for (int k = 0; k < 3; k++)
-            {
-                V3 dp = v3(0.f, 0.f, 0.f);
-                if (g.positions)
+                const V3 dNraw = normalize_grad(t.Nn, t.nlen, dNn);
+                dl = normalize_grad(t.L, t.llen, dL);
+                // P, N, A = sum b_k (p_k, n_k, a_k)
+                float db[3];
+                for (int k = 0; k < 3; k++)
+                    db[k] = dot(dP, s.p[k]) + dot(dNraw, s.n[k]) + dot(dA, s.a[k]);
+                // b = bt / S
+                const float bdb = s.b[0] * db[0] + s.b[1] * db[1] + s.b[2] * db[2];
+                float dbt[3];
+                for (int k = 0; k < 3; k++)
+                    dbt[k] = (db[k] - bdb) / s.S;
+                // bt = a x c
+                float dac[3] = { 0.f, 0.f, 0.f }, dcc[3] = { 0.f, 0.f, 0.f };
+                dac[1] += dbt[0] * s.cc[2]; dcc[2] += dbt[0] * s.ac[1]; dac[2] -= dbt[0] * s.cc[1]; dcc[1] -= dbt[0] * s.ac[2];
+                dac[2] += dbt[1] * s.cc[0]; dcc[0] += dbt[1] * s.ac[2]; dac[0] -= dbt[1] * s.cc[2]; dcc[2] -= dbt[1] * s.ac[0];
+                dac[0] += dbt[2] * s.cc[1]; dcc[1] += dbt[2] * s.ac[0]; dac[1] -= dbt[2] * s.cc[0]; dcc[0] -= dbt[2] * s.ac[1];
+                // a_k = X_k - u W_k, c_k = Y_k - v W_k, (X, Y, W) = rows 0, 1, 3 of MVP (p, 1)
+                for (int k = 0; k < 3; k++)
                 {
-                    const float dX = dac[k], dY = dcc[k], dW = -s.u * dac[k] - s.v * dcc[k];
-                    const float* M = f.mvp;
-                    dp = v3(M[0] * dX + M[4] * dY + M[12] * dW, M[1] * dX + M[5] * dY + M[13] * dW,
-                            M[2] * dX + M[6] * dY + M[14] * dW);
-                    dp = dp + s.b[k] * dP;
-                }
-                if (Packed)
-                    add_packed(g.packed, s.vi[k], s.b[k] * dA, s.b[k] * dNraw, dp);
-                else
-                {
-                    add3(g.albedo, s.vi[k], s.b[k] * dA);
-                    add3(g.normals, s.vi[k], s.b[k] * dNraw);
-                    add3(g.positions, s.vi[k], dp);
+                    V3 dp = v3(0.f, 0.f, 0.f);
+                    if (g.positions)
+                    {
+                        const float dX = dac[k], dY = dcc[k], dW = -s.u * dac[k] - s.v * dcc[k];
+                        const float* M = f.mvp;
+                        dp = v3(M[0] * dX + M[4] * dY + M[12] * dW, M[1] * dX + M[5] * dY + M[13] * dW,
+                                M[2] * dX + M[6] * dY + M[14] * dW);
+                        dp = dp + s.b[k] * dP;
+                    }
+                    if (Packed)
+                        add_packed(g.packed, s.vi[k], s.b[k] * dA, s.b[k] * dNraw, dp);
+                    else
+                    {
+                        add3(g.albedo, s.vi[k], s.b[k] * dA);
+                        add3(g.normals, s.vi[k], s.b[k] * dNraw);
+                        add3(g.positions, s.vi[k], dp);
+                    }
                 }
             }
         }
-    }
-    // block-reduce the five global gradients together (one barrier),
-    // accumulate in double
-    float vals[5] = { dl.x, dl.y, dl.z, dks, dshin };
+        // the five global gradients: summed over the warp, then in double
+        float vals[5] = { dl.x, dl.y, dl.z, dks, dshin };
 #pragma unroll
-    for (int q = 0; q < 5; q++)
-        for (int o = 16; o > 0; o >>= 1)
-            vals[q] += __shfl_down_sync(0xffffffffu, vals[q], o);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        for (int q = 0; q < 5; q++)
+        {
+            for (int o = 16; o > 0; o >>= 1)
+                vals[q] += __shfl_down_sync(0xffffffffu, vals[q], o);
+            if (lane == 0)
+                sums[q] += (double)vals[q];
+        }
+    }
     if (lane == 0)
 #pragma unroll
         for (int q = 0; q < 5; q++)
-            red[q * (kThreads / 32) + warp] = vals[q];
+            red[warp][q] = sums[q];
     __syncthreads();
-    if (warp == 0)
+    if (threadIdx.x < 5)
     {
-#pragma unroll
-        for (int q = 0; q < 5; q++)
-        {
-            float r = lane < kThreads / 32 ? red[q * (kThreads / 32) + lane] : 0.0f;
-            for (int o = 16; o > 0; o >>= 1)
-                r += __shfl_down_sync(0xffffffffu, r, o);
-            if (lane == 0 && r != 0.0f)
-                atomicAdd(g.scratch + q, (double)r);
-        }
+        double r = 0.0;
+        for (int w = 0; w < kWarps; w++)
+            r += red[w][threadIdx.x];
+        if (r != 0.0)
+            atomicAdd(g.scratch + threadIdx.x, r);
     }
 }
 
@@ -467,21 +527,32 @@ __global__ void __launch_bounds__(kThreads) k_finish(DiffGrads g, uint32_t nv)
 
 }  // namespace
 
+// Rows of 32 pixels per warp: as many as leave each SM about 48 warps of
+// work, so that small images still spread over the chip.
+static int span_rows(const PassArgs& a, uint64_t total)
+{
+    const uint64_t sms = a.num_sms > 0 ? (uint64_t)a.num_sms : 148, rows = total / (32 * 48 * sms);
+    return rows < 1 ? 1 : rows > kSpan / 32 ? kSpan / 32 : (int)rows;
+}
+
 cudaError_t launch_shade_visible(const PassArgs& a, uint64_t total, const DiffMesh& m, float4* out, cudaStream_t s)
 {
+    const int rows = span_rows(a, total);
     if (total)
-        k_shade_visible<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, s>>>(a, total, m, out);
+        k_shade_visible<<<(unsigned)((total + kThreads * rows - 1) / (kThreads * rows)), kThreads, 0, s>>>(a, total, rows,
+                                                                                                          m, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_backward(const PassArgs& a, uint64_t total, const DiffMesh& m, const float4* grad,
                             const DiffGrads& g, cudaStream_t s)
 {
-    const unsigned blocks = (unsigned)((total + kThreads - 1) / kThreads);
+    const int rows = span_rows(a, total);
+    const unsigned blocks = (unsigned)((total + kThreads * rows - 1) / (kThreads * rows));
     if (total && g.packed)
-        k_backward<true><<<blocks, kThreads, 0, s>>>(a, total, m, grad, g);
+        k_backward<true><<<blocks, kThreads, 0, s>>>(a, total, rows, m, grad, g);
     else if (total)
-        k_backward<false><<<blocks, kThreads, 0, s>>>(a, total, m, grad, g);
+        k_backward<false><<<blocks, kThreads, 0, s>>>(a, total, rows, m, grad, g);
     k_finish<<<g.packed ? (m.nv + kThreads - 1) / kThreads : 1, kThreads, 0, s>>>(g, m.nv);
     return cudaGetLastError();
 }
