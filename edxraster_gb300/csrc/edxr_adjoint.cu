@@ -76,54 +76,6 @@ __device__ __forceinline__ V3 ld(const char* base, uint32_t stride, uint32_t i, 
 // gradient of normalize(x) applied to dy: (dy - y (y . dy)) / |x|
 __device__ __forceinline__ V3 normalize_grad(V3 y, float lenx, V3 dy) { return (1.0f / lenx) * (dy - dot(y, dy) * y); }
 
-// Float pairs: the value hi + lo, |lo| <= ulp(hi) / 2.
-struct FF
-{
-    float hi, lo;
-};
-// a * b exactly, as a pair (needs the product rounded once: the library is
-// built without contraction, and fmaf gives the exact remainder).
-__device__ __forceinline__ FF two_prod(float a, float b)
-{
-    const float p = a * b;
-    return { p, fmaf(a, b, -p) };
-}
-// a + b exactly, as a pair.
-__device__ __forceinline__ FF two_sum(float a, float b)
-{
-    const float s = a + b;
-    const float bb = s - a;
-    return { s, (a - (s - bb)) + (b - bb) };
-}
-__device__ __forceinline__ FF quick_two_sum(float a, float b)  // |a| >= |b|
-{
-    const float s = a + b;
-    return { s, b - (s - a) };
-}
-// The pairs below are summed with the errors of the additions and products
-// gathered in the low part and renormalised once at the end (the low parts
-// stay around the rounding errors of the high ones), which takes about a
-// quarter fewer instructions than renormalising after every operation and
-// loses nothing that shows in the rounded results.
-// x + y, not renormalised.
-__device__ __forceinline__ FF ff_sum(FF x, FF y)
-{
-    const FF s = two_sum(x.hi, y.hi);
-    return { s.hi, s.lo + (x.lo + y.lo) };
-}
-// x * y, not renormalised.
-__device__ __forceinline__ FF ff_prod(FF x, FF y)
-{
-    const FF p = two_prod(x.hi, y.hi);
-    return { p.hi, fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, p.lo)) };
-}
-__device__ __forceinline__ FF ff_prod_f(FF x, float y)
-{
-    const FF p = two_prod(x.hi, y);
-    return { p.hi, fmaf(x.lo, y, p.lo) };
-}
-__device__ __forceinline__ FF ff_neg(FF x) { return { -x.hi, -x.lo }; }
-__device__ __forceinline__ FF ff_norm(FF x) { return quick_two_sum(x.hi, x.lo); }
 // m0 x + m1 y + m2 z + m3 as a pair.
 __device__ __forceinline__ FF ff_dot4(float m0, float m1, float m2, float m3, float x, float y, float z)
 {

