@@ -509,12 +509,11 @@ edxr_status launch_frames(edxr_renderer* r, uint32_t n, uint32_t width, uint32_t
     if (vertex_stage)
         EDXR_CUDA(r->vrecs.ensure(sizeof(int4) * tv));
 
-    EDXR_CUDA(cudaMemcpyAsync(r->frames.ptr, r->frames_host, sizeof(FrameDesc) * n, cudaMemcpyHostToDevice, r->stream));
-
     PassArgs a;
     std::memset(&a, 0, sizeof(a));
     a.tune = r->tuning;
     a.frames = r->frames.as<FrameDesc>();
+    a.frames_host = r->frames_host;
     a.num_frames = n;
     a.tiles_per_frame = equal_tiles && n > 1 ? (uint32_t)(tiles / n) : 0u;  // (one frame: no search)
     if (n > 1)
@@ -544,6 +543,7 @@ edxr_status launch_frames(edxr_renderer* r, uint32_t n, uint32_t width, uint32_t
     a.counters = r->counters.as<uint32_t>();
     a.scan_status = reinterpret_cast<unsigned long long*>(a.counters + kCounters);
     a.status = r->status.as<DeviceStatus>();
+    a.status_host = r->status_host;
     a.color = r->color.as<float4>();
     a.depth = r->depth.as<float>();
     a.tri_id = r->tri_id.as<uint32_t>();
@@ -557,7 +557,6 @@ edxr_status launch_frames(edxr_renderer* r, uint32_t n, uint32_t width, uint32_t
     a.num_sms = r->num_sms;
 
     EDXR_CUDA(run_pass(r, a));
-    EDXR_CUDA(cudaMemcpyAsync(r->status_host, r->status.ptr, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, r->stream));
     EDXR_CUDA(cudaEventRecord(r->done, r->stream));
     r->last = a;
     r->pending = true;
@@ -649,7 +648,6 @@ edxr_status sync_pass(edxr_renderer* r)
         }
         r->rerenders++;
         EDXR_CUDA(run_pass(r, a));
-        EDXR_CUDA(cudaMemcpyAsync(r->status_host, r->status.ptr, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, r->stream));
         EDXR_CUDA(cudaEventRecord(r->done, r->stream));
         r->last = a;
     }

@@ -160,6 +160,7 @@ struct PassArgs
 {
     Tuning tune;
     const FrameDesc* frames;
+    const FrameDesc* frames_host;  // page-locked: copied to `frames` at the start of the pass, or NULL
     uint32_t num_frames;
     uint32_t tiles_per_frame;  // every frame's tile count when they are equal (then frame = tile / it), else 0
     uint32_t* frame_of_block;  // several frames: the frame of triangle 256 b, per b (filled by k_clear); else NULL
@@ -196,6 +197,7 @@ struct PassArgs
     uint32_t* empty_tiles;   // the tiles with no bin entry (counters[9] of them), total_tiles words
     unsigned long long* keybuf;  // per pixel: ~(smallest key) of split tiles, 0 between passes
     DeviceStatus* status;
+    DeviceStatus* status_host;  // page-locked copy that the raster kernel writes, or NULL
     uint32_t* tri_first;     // per clipped input triangle: its first fan piece
     float4* color;
     float* depth;

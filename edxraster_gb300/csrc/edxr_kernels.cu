@@ -25,6 +25,17 @@ constexpr uint32_t kBigChunk = 128;    // unsorted-list slots a k_bin_big warp r
 constexpr uint32_t kEmptySlot = 0xFFFFFFFFu;
 constexpr uint32_t kSplitTile = 0x80000000u;  // item tag: the tile has several items (tiles < 2^24)
 
+// Programmatic dependent launch: the pass's kernels follow one another with the
+// next one's blocks already resident.  Each kernel first lets its successor be
+// scheduled (which happens once all of its own blocks run) and then waits for
+// its predecessor's end and memory; nothing is read or written before the
+// wait.  A kernel so starts about a microsecond after its predecessor's last
+// block instead of two.
+__device__ __forceinline__ void follow_on()
+{
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+
 // Clip-space position of vertex v: clip = MVP * (p, 1) (DefaultVertexShader,
 // Shader.h:40-49).
 __device__ __forceinline__ float4 clip_position(const FrameDesc& f, uint32_t v)
@@ -55,6 +66,7 @@ __device__ __forceinline__ int4 vertex_record(const FrameDesc& f, uint32_t v)
 // Clear of the per-tile counters and work queues, and the vertex stage.
 __global__ void k_clear(PassArgs a)
 {
+    follow_on();
     const uint32_t stride = gridDim.x * blockDim.x;
     if (a.vrecs)
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.total_vertices; i += stride)
@@ -251,6 +263,7 @@ __device__ __forceinline__ uint32_t frame_of_triangle(const PassArgs& a, uint32_
 // stripe of the unsorted bin list take one atomic per warp each.
 __global__ void __launch_bounds__(256, 6) k_setup(PassArgs a)
 {
+    follow_on();
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31;
     uint32_t fi = 0, tri = 0;
@@ -728,6 +741,7 @@ __device__ __forceinline__ void clip_lanes(const PassArgs& a, uint32_t nq, float
 
 __global__ void __launch_bounds__(kClipThreads) k_clip(PassArgs a)
 {
+    follow_on();
     __shared__ float4 s_vc[kClipWarps][kClipPer][kMaxPolygon];
     const uint32_t nq = min(*(volatile uint32_t*)&a.counters[4], a.poly_capacity);
     if (nq <= gridDim.x * (uint32_t)(kClipThreads / kClipLanes))
@@ -741,6 +755,7 @@ __global__ void __launch_bounds__(kClipThreads) k_clip(PassArgs a)
 // bin holds its tile's first tile_cursor entries.
 __global__ void __launch_bounds__(256) k_bin_move(PassArgs a)
 {
+    follow_on();
     // the filled parts of the stripes (slots past a stripe's end were
     // dropped: overflow), numbered one after another
     __shared__ uint32_t s_first[kBinStripes + 1];
@@ -854,6 +869,7 @@ __device__ __forceinline__ uint32_t zmax_key(const RTri& t)
 // it leaves unused are marked empty.
 __global__ void __launch_bounds__(256, 4) k_bin_big(PassArgs a)
 {
+    follow_on();
     const uint32_t nb = min(*(volatile uint32_t*)&a.counters[2], a.big_capacity);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -1035,6 +1051,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* warp_sums, 
 
 __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
 {
+    follow_on();
     __shared__ uint32_t warp_sums[33];
     __shared__ uint32_t s_block, s_prefix;
     if (threadIdx.x == 0)
@@ -1558,6 +1575,14 @@ static __device__ __forceinline__ void clear_tile(const PassArgs& a, uint32_t ti
     }
 }
 
+// The pass's status word, final once the raster kernel runs, written to the
+// host (page-locked memory) by its first thread: no copy follows the pass.
+__device__ __forceinline__ void report_status(const PassArgs& a)
+{
+    if (a.status_host && blockIdx.x == 0 && threadIdx.x == 0)
+        *a.status_host = *a.status;
+}
+
 // Barrier of the Group warps that share an item: the warp's own lanes
 // (Group 1), the whole block (Group 8), or a named barrier per group.
 template <int Group>
@@ -1596,12 +1621,14 @@ __device__ __forceinline__ void lower_key(unsigned long long* slot, unsigned lon
 template <int Group>
 __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
 {
+    follow_on();
     constexpr int kGroups = kRasterWarps / Group;   // groups of a block
     constexpr int kThreads = 32 * Group;            // threads of a group
     constexpr int kPixels = 256 / kThreads;         // pixels of the tile per thread
     __shared__ unsigned long long s_key[kGroups][256];
     __shared__ StagedSlot s_tri[kRasterWarps][32];
     __shared__ uint32_t s_next[kGroups], s_done[kGroups];
+    report_status(a);
     if (*(volatile uint32_t*)&a.status->error)
         return;  // the pass failed (see k_bin_move); every thread of the block leaves
     // ceil(65536 / w): ((p * s_recip[w]) >> 16) == p / w for 0 <= p < 256 and
@@ -2141,10 +2168,12 @@ __host__ __device__ constexpr int ms_blocks(int S) { return S <= 8 ? 8 : 3; }
 template <int S>
 __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(const __grid_constant__ PassArgs a)
 {
+    follow_on();
     constexpr int W = ms_warps(S);
     constexpr int kThreads = 32 * W;
     extern __shared__ unsigned long long ms_shared[];
     __shared__ uint32_t s_next, s_done, s_bound[W];
+    report_status(a);
     if (*(volatile uint32_t*)&a.status->error)
         return;  // the pass failed (see k_bin_move); every thread of the block leaves
     // ceil(65536 / w): ((p * s_recip[w]) >> 16) == p / w for 0 <= p < 256
@@ -2459,13 +2488,32 @@ static int raster_occupancy()
     return per_sm;
 }
 
+// Launches a kernel of the pass; `follows`: right behind the pass's previous
+// kernel (see follow_on).
+template <typename Kernel>
+static cudaError_t launch(Kernel kernel, unsigned blocks, unsigned threads, size_t smem, cudaStream_t s, bool follows,
+                          const PassArgs& a)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = follows ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, a);
+}
+
 template <int Group>
-static void launch_raster(int sms, const PassArgs& a, cudaStream_t s)
+static cudaError_t launch_raster(int sms, const PassArgs& a, cudaStream_t s, bool follows)
 {
     int per = raster_occupancy<Group>();
     if (a.tune.raster_blocks_per_sm > 0 && a.tune.raster_blocks_per_sm < per)
         per = a.tune.raster_blocks_per_sm;
-    k_raster<Group><<<sms * per, kRasterThreads, 0, s>>>(a);
+    return launch(k_raster<Group>, (unsigned)(sms * per), kRasterThreads, 0, s, follows, a);
 }
 
 // Warps per raster item.  A warp alone takes 10 to 25 us for a tile (a chain
@@ -2560,48 +2608,61 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
     };
+    cudaError_t e = cudaSuccess;
+    // (stage events between the kernels keep them apart)
+    bool follows = false;
+    auto go = [&](auto kernel, uint64_t blocks, unsigned threads, size_t smem) {
+        if (e == cudaSuccess)
+            e = launch(kernel, (unsigned)blocks, threads, smem, s, follows, a);
+        follows = !ev;
+    };
+    if (a.frames_host)
+        e = cudaMemcpyAsync(const_cast<FrameDesc*>(a.frames), a.frames_host, sizeof(FrameDesc) * a.num_frames,
+                            cudaMemcpyHostToDevice, s);
     mark(0);
     const uint32_t clear_items = max(a.total_tiles + 1, a.vrecs ? a.total_vertices : 0u);
-    k_clear<<<(clear_items + 255) / 256 + 1, 256, 0, s>>>(a);
+    go(k_clear, (clear_items + 255) / 256 + 1, 256, 0);
     mark(1);
     if (a.total_tris)
     {
-        k_setup<<<(a.total_tris + 255) / 256, 256, 0, s>>>(a);
-        k_clip<<<sms * 8, kClipThreads, 0, s>>>(a);
+        go(k_setup, (a.total_tris + 255) / 256, 256, 0);
+        go(k_clip, sms * 8, kClipThreads, 0);
     }
-    k_bin_big<<<sms * 4, 256, 0, s>>>(a);
+    go(k_bin_big, sms * 4, 256, 0);
     mark(2);
-    k_scan<<<nscan, kScanThreads, 0, s>>>(a);
+    go(k_scan, nscan, kScanThreads, 0);
     mark(3);
-    k_bin_move<<<sms * (a.tune.bin_blocks_per_sm > 0 ? a.tune.bin_blocks_per_sm : 8), 256, 0, s>>>(a);
+    go(k_bin_move, sms * (a.tune.bin_blocks_per_sm > 0 ? a.tune.bin_blocks_per_sm : 8), 256, 0);
     mark(4);
     if (a.msaa_log2 > 0)
     {
         const int level = min(a.msaa_log2, kMaxMsaaLog2), S = 1 << level;
-        const int blocks = sms * ms_occupancy(level), threads = 32 * ms_warps(S);
+        const unsigned blocks = (unsigned)(sms * ms_occupancy(level)), threads = 32u * (unsigned)ms_warps(S);
         switch (level)
         {
-        case 1: k_raster_ms<2><<<blocks, threads, ms_smem(2), s>>>(a); break;
-        case 2: k_raster_ms<4><<<blocks, threads, ms_smem(4), s>>>(a); break;
-        case 3: k_raster_ms<8><<<blocks, threads, ms_smem(8), s>>>(a); break;
-        case 4: k_raster_ms<16><<<blocks, threads, ms_smem(16), s>>>(a); break;
-        default: k_raster_ms<32><<<blocks, threads, ms_smem(32), s>>>(a); break;
+        case 1: go(k_raster_ms<2>, blocks, threads, ms_smem(2)); break;
+        case 2: go(k_raster_ms<4>, blocks, threads, ms_smem(4)); break;
+        case 3: go(k_raster_ms<8>, blocks, threads, ms_smem(8)); break;
+        case 4: go(k_raster_ms<16>, blocks, threads, ms_smem(16)); break;
+        default: go(k_raster_ms<32>, blocks, threads, ms_smem(32)); break;
         }
     }
-    else
+    else if (e == cudaSuccess)
     {
+        const int group = raster_group(a, sms);
         if (a.tune.raster_variant == 2)
             a.tune.small_region = 0;
-        switch (raster_group(a, sms))
+        switch (group)
         {
-        case 8: launch_raster<8>(sms, a, s); break;
-        case 4: launch_raster<4>(sms, a, s); break;
-        case 2: launch_raster<2>(sms, a, s); break;
-        default: launch_raster<1>(sms, a, s); break;
+        case 8: e = launch_raster<8>(sms, a, s, follows); break;
+        case 4: e = launch_raster<4>(sms, a, s, follows); break;
+        case 2: e = launch_raster<2>(sms, a, s, follows); break;
+        default: e = launch_raster<1>(sms, a, s, follows); break;
         }
     }
     mark(5);
-    return cudaGetLastError();
+    const cudaError_t last = cudaGetLastError();
+    return e != cudaSuccess ? e : last;
 }
 
 int kernels_per_pass(const PassArgs& a)
