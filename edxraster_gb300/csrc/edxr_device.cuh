@@ -473,15 +473,19 @@ struct ShadeVerts
 
 // Attributes of the raster vertices of triangle t (Clipper.h:138-151 for the
 // vertices the clipper created: weight.x*a0 + weight.y*a1 + weight.z*a2).
+// NormalsOnly: positions and albedo are not read (the textured shader).
+template <bool NormalsOnly = false>
 __device__ __forceinline__ ShadeVerts shade_verts(const FrameDesc& f, const RTri& t, const ClipPoly* polys)
 {
     const uint32_t tri = t.order >> 4;
     const uint32_t i0 = __ldg(f.indices + 3 * (size_t)tri + 0);
     const uint32_t i1 = __ldg(f.indices + 3 * (size_t)tri + 1);
     const uint32_t i2 = __ldg(f.indices + 3 * (size_t)tri + 2);
-    float3 sp[3] = { ld3(f.positions, f.pos_stride, i0, 0.f), ld3(f.positions, f.pos_stride, i1, 0.f), ld3(f.positions, f.pos_stride, i2, 0.f) };
+    const char* pos = NormalsOnly ? nullptr : f.positions;
+    const char* alb = NormalsOnly ? nullptr : f.albedo;
+    float3 sp[3] = { ld3(pos, f.pos_stride, i0, 0.f), ld3(pos, f.pos_stride, i1, 0.f), ld3(pos, f.pos_stride, i2, 0.f) };
     float3 sn[3] = { ld3(f.normals, f.nrm_stride, i0, 0.f), ld3(f.normals, f.nrm_stride, i1, 0.f), ld3(f.normals, f.nrm_stride, i2, 0.f) };
-    float3 sa[3] = { ld3(f.albedo, f.alb_stride, i0, 1.f), ld3(f.albedo, f.alb_stride, i1, 1.f), ld3(f.albedo, f.alb_stride, i2, 1.f) };
+    float3 sa[3] = { ld3(alb, f.alb_stride, i0, 1.f), ld3(alb, f.alb_stride, i1, 1.f), ld3(alb, f.alb_stride, i2, 1.f) };
     ShadeVerts v;
     if (t.poly == kUnclipped)
     {
@@ -954,8 +958,9 @@ static __device__ __noinline__ float3 shade_fragment_pairs(const FrameDesc& f, c
     return f3(c.hi, c.hi, c.hi);
 }
 
-// Fragment::Interpolate (Shader.h:142-170) from the fragment's barycentrics,
-// then the shading model.
+// The reference Blinn-Phong shader or the textured one (the others are
+// shade_common): Fragment::Interpolate (Shader.h:142-170) from the fragment's
+// barycentrics, then the shading model.
 // t is the record at tg (global memory).
 __device__ __forceinline__ float3 shade_fragment(const FrameDesc& f, const RTri& t, const RTri* tg,
                                                  const ClipPoly* polys, float l0, float l1, int px, int py)
@@ -971,11 +976,9 @@ __device__ __forceinline__ float3 shade_fragment(const FrameDesc& f, const RTri&
     b0 = fmul(b0, invB);
     b1 = fmul(b1, invB);
     b2 = fsub(fsub(1.0f, b0), b1);
-    const ShadeVerts v = shade_verts(f, t, polys);
-    const float3 P = lerp3(b0, v.p[0], b1, v.p[1], b2, v.p[2]);
-    const float3 N = lerp3(b0, v.n[0], b1, v.n[1], b2, v.n[2]);
-    const float3 A = f.ps_kind == 4 ? texture_albedo(f, tg, polys, px, py) : lerp3(b0, v.a[0], b1, v.a[1], b2, v.a[2]);
-    return shade_model(f, P, N, A);
+    const ShadeVerts v = shade_verts<true>(f, t, polys);
+    return shade_model(f, f3(0.f, 0.f, 0.f), lerp3(b0, v.n[0], b1, v.n[1], b2, v.n[2]),
+                       texture_albedo(f, tg, polys, px, py));
 }
 
 // Frame owning output pixel i (binary search over pix_base).

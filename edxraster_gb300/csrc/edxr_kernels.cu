@@ -1552,12 +1552,9 @@ __device__ __forceinline__ unsigned long long depth_key64(int l1, int l2, const 
 }
 
 // The background of a tile, written by `threads` threads.
-static __device__ __forceinline__ void clear_tile(const PassArgs& a, uint32_t tile, int thread, int threads)
+static __device__ __forceinline__ void clear_tile(const PassArgs& a, const FrameDesc& f, uint32_t tile, int thread,
+                                                  int threads)
 {
-    const uint32_t fi = a.tiles_per_frame ? tile / a.tiles_per_frame
-                                          : find_frame(a.frames, a.num_frames, tile,
-                                                       [](const FrameDesc& f) { return f.tile_base; });
-    const FrameDesc& f = a.frames[fi];
     const uint32_t lt = tile - f.tile_base;
     const int tileX = (int)(lt % (uint32_t)f.tdx), tileY = (int)(lt / (uint32_t)f.tdx);
     const int w = f.width, h = f.height;
@@ -1618,7 +1615,7 @@ __device__ __forceinline__ void lower_key(unsigned long long* slot, unsigned lon
 // instead of 217 on the binning stress (3840x2160), 67 instead of 55 on a
 // 301x301-quad terrain at 1366x769; at 4 blocks 109, 219 and 61; at 2 blocks
 // (124 registers) 111, 250 and 53.
-template <int Group>
+template <int Group, bool One>
 __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
 {
     follow_on();
@@ -1634,6 +1631,14 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
     // ceil(65536 / w): ((p * s_recip[w]) >> 16) == p / w for 0 <= p < 256 and
     // 1 <= w <= 16, the row of pixel p of a region w pixels wide
     __shared__ uint32_t s_recip[17];
+    // A pass of one frame (One) keeps its descriptor in shared memory: the
+    // shading reads some twenty of its fields a pixel, and stores to the images
+    // keep the compiler from holding them (raster stage: terrain 95 -> 93 us,
+    // binning stress 219 -> 211).
+    __shared__ FrameDesc s_frame;
+    if (One)
+        for (int k = (int)threadIdx.x; k < (int)(sizeof(FrameDesc) / 8); k += kRasterThreads)
+            reinterpret_cast<unsigned long long*>(&s_frame)[k] = reinterpret_cast<const unsigned long long*>(a.frames)[k];
     if (threadIdx.x >= 1 && threadIdx.x <= 16)
         s_recip[threadIdx.x] = (65536u + threadIdx.x - 1u) / threadIdx.x;
     __syncthreads();
@@ -1664,6 +1669,14 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
     const uint32_t shared_tiles = share * nitems;
     const uint32_t bulk = min(8u, max(1u, (nempty - shared_tiles) / ngroups));
     const uint32_t nwork = nitems + (nempty - shared_tiles + bulk - 1) / bulk;
+    // the frame of a tile
+    auto frame_of = [&](uint32_t tile) -> const FrameDesc& {
+        if (One)
+            return s_frame;
+        return a.frames[a.tiles_per_frame ? tile / a.tiles_per_frame
+                                          : find_frame(a.frames, a.num_frames, tile,
+                                                       [](const FrameDesc& f) { return f.tile_base; })];
+    };
     auto next_item = [&]() -> uint32_t {
         if (ngroups >= nwork)
             return nwork;
@@ -1680,19 +1693,16 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
         {
             const uint32_t i0 = shared_tiles + (q - nitems) * bulk, i1 = min(nempty, i0 + bulk);
             for (uint32_t i = i0; i < i1; i++)
-                clear_tile(a, a.empty_tiles[i], gthread, kThreads);
+                clear_tile(a, frame_of(a.empty_tiles[i]), a.empty_tiles[i], gthread, kThreads);
             if (Group > 1)
                 group_sync<Group>(group);
             continue;
         }
         const uint4 item = a.items[q < nheavy ? q : (uint32_t)(a.item_capacity - 1 - (q - nheavy))];
         for (uint32_t i = 0; i < share; i++)
-            clear_tile(a, a.empty_tiles[q * share + i], gthread, kThreads);
+            clear_tile(a, frame_of(a.empty_tiles[q * share + i]), a.empty_tiles[q * share + i], gthread, kThreads);
         const uint32_t tile = item.x & ~kSplitTile;
-        const uint32_t fi = a.tiles_per_frame ? tile / a.tiles_per_frame
-                                              : find_frame(a.frames, a.num_frames, tile,
-                                                           [](const FrameDesc& f) { return f.tile_base; });
-        const FrameDesc& f = a.frames[fi];
+        const FrameDesc& f = frame_of(tile);
         const uint32_t lt = tile - f.tile_base;
         const int tileX = (int)(lt % (uint32_t)f.tdx), tileY = (int)(lt / (uint32_t)f.tdx);
         const bool less = f.depth_func == 1;
@@ -1724,7 +1734,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
         if (e0 == e1 && !split)
         {
             // every entry was hidden behind the clear depth: the background, with no key
-            clear_tile(a, tile, gthread, kThreads);
+            clear_tile(a, f, tile, gthread, kThreads);
             if (Group > 1)
                 group_sync<Group>(group);
             continue;
@@ -2115,12 +2125,9 @@ static __device__ __noinline__ void shade_tile_ms_slow(const PassArgs& a, const 
 
 // The background of a tile with S samples, written by `threads` threads.
 template <int S>
-static __device__ __forceinline__ void clear_tile_ms(const PassArgs& a, uint32_t tile, int thread, int threads)
+static __device__ __forceinline__ void clear_tile_ms(const PassArgs& a, const FrameDesc& f, uint32_t tile, int thread,
+                                                     int threads)
 {
-    const uint32_t fi = a.tiles_per_frame ? tile / a.tiles_per_frame
-                                          : find_frame(a.frames, a.num_frames, tile,
-                                                       [](const FrameDesc& f) { return f.tile_base; });
-    const FrameDesc& f = a.frames[fi];
     const uint32_t lt = tile - f.tile_base;
     const int tileX = (int)(lt % (uint32_t)f.tdx), tileY = (int)(lt / (uint32_t)f.tdx);
     const int w = f.width, h = f.height;
@@ -2179,6 +2186,11 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
     // ceil(65536 / w): ((p * s_recip[w]) >> 16) == p / w for 0 <= p < 256
     // and 1 <= w <= 16, the row of pixel p of a region w pixels wide
     __shared__ uint32_t s_recip[17];
+    // (several samples: one frame, its descriptor as in k_raster)
+    __shared__ FrameDesc s_frame;
+    for (int k = (int)threadIdx.x; k < (int)(sizeof(FrameDesc) / 8); k += kThreads)
+        reinterpret_cast<unsigned long long*>(&s_frame)[k] = reinterpret_cast<const unsigned long long*>(a.frames)[k];
+    const FrameDesc& f = s_frame;
     if (threadIdx.x >= 1 && threadIdx.x <= 16)
         s_recip[threadIdx.x] = (65536u + threadIdx.x - 1u) / threadIdx.x;
     __syncthreads();
@@ -2214,16 +2226,12 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
         {
             const uint32_t i0 = (q - nitems) * bulk, i1 = min(nempty, i0 + bulk);
             for (uint32_t i = i0; i < i1; i++)
-                clear_tile_ms<S>(a, a.empty_tiles[i], (int)threadIdx.x, kThreads);
+                clear_tile_ms<S>(a, f, a.empty_tiles[i], (int)threadIdx.x, kThreads);
             __syncthreads();
             continue;
         }
         const uint4 item = a.items[q < nheavy ? q : (uint32_t)(a.item_capacity - 1 - (q - nheavy))];
         const uint32_t tile = item.x & ~kSplitTile;
-        const uint32_t fi = a.tiles_per_frame ? tile / a.tiles_per_frame
-                                              : find_frame(a.frames, a.num_frames, tile,
-                                                           [](const FrameDesc& f) { return f.tile_base; });
-        const FrameDesc& f = a.frames[fi];
         const uint32_t lt = tile - f.tile_base;
         const int tileX = (int)(lt % (uint32_t)f.tdx), tileY = (int)(lt / (uint32_t)f.tdx);
         const bool less = f.depth_func == 1;
@@ -2251,7 +2259,7 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
         if (e0 == e1 && !split)
         {
             // every entry was hidden behind the clear depth: the background, with no key
-            clear_tile_ms<S>(a, tile, (int)threadIdx.x, kThreads);
+            clear_tile_ms<S>(a, f, tile, (int)threadIdx.x, kThreads);
             __syncthreads();
             continue;
         }
@@ -2481,7 +2489,7 @@ static int raster_occupancy()
     if (!per_sm)
     {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_raster<Group>, kRasterThreads, 0) != cudaSuccess || n < 1)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_raster<Group, false>, kRasterThreads, 0) != cudaSuccess || n < 1)
             n = 1;
         per_sm = n;
     }
@@ -2513,7 +2521,7 @@ static cudaError_t launch_raster(int sms, const PassArgs& a, cudaStream_t s, boo
     int per = raster_occupancy<Group>();
     if (a.tune.raster_blocks_per_sm > 0 && a.tune.raster_blocks_per_sm < per)
         per = a.tune.raster_blocks_per_sm;
-    return launch(k_raster<Group>, (unsigned)(sms * per), kRasterThreads, 0, s, follows, a);
+    return launch((a.num_frames == 1 ? k_raster<Group, true> : k_raster<Group, false>), (unsigned)(sms * per), kRasterThreads, 0, s, follows, a);
 }
 
 // Warps per raster item.  A warp alone takes 10 to 25 us for a tile (a chain
