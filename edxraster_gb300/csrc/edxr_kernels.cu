@@ -1054,6 +1054,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
     follow_on();
     __shared__ uint32_t warp_sums[33];
     __shared__ uint32_t s_block, s_prefix;
+    __shared__ bool s_dropped;
+    const uint32_t lane = threadIdx.x & 31;
     if (threadIdx.x == 0)
         s_block = atomicAdd(&a.counters[8], 1u);
     __syncthreads();
@@ -1067,45 +1069,65 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
         cnt[k] = (i < a.total_tiles) ? a.tile_count[i] : 0u;
         sum += padded(cnt[k]);
     }
+    // (the last warp, for the statistics as well; loaded before the scan's
+    // barriers and the look-back)
+    uint32_t filled = 0, survived = 0;
+    if (threadIdx.x >= kScanThreads - 32)
+    {
+        static_assert(kBinStripes == 32, "one lane per stripe");
+        const volatile uint32_t* c = stripe_counter(a, lane);
+        filled = c[0];
+        survived = c[1];
+        const bool over = __any_sync(0xffffffffu, filled > stripe_slots(a.bin_capacity));
+        if (lane == 0)
+            s_dropped = over;
+    }
     uint32_t total;
     const uint32_t incl = block_scan(sum, warp_sums, total);
-    if (threadIdx.x == 0)
+    // Look back over the ranges before this one, a warp's lanes on 32 of them
+    // at a time: the nearest that publishes everything up to its end, and the
+    // sums of those after it.  (One thread walking them took an L2 round trip
+    // per range.)
+    if (threadIdx.x < 32)
     {
-        uint32_t prefix = 0;
         // (a failure test makes one block keep its sums to itself)
-        const bool publish = (int)b != a.tune.scan_stall_block;
+        const bool publish = (int)b != a.tune.scan_stall_block && lane == 0;
         const int spin_limit = a.tune.scan_spin_limit > 0 ? a.tune.scan_spin_limit : kScanSpinLimit;
-        if (b == 0)
+        uint32_t prefix = 0;
+        if (b > 0 && publish)
+            atomicExch(&a.scan_status[b], kScanAggregate | total);
+        for (int j = (int)b - 1, spins = 0; j >= 0;)
         {
-            if (publish)
-                atomicExch(&a.scan_status[0], kScanPrefix | total);
-        }
-        else
-        {
-            if (publish)
-                atomicExch(&a.scan_status[b], kScanAggregate | total);
-            for (int j = (int)b - 1; j >= 0;)
+            const int r = j - (int)lane;
+            unsigned long long st = kScanPrefix;
+            if (r >= 0)
+                st = *(volatile unsigned long long*)&a.scan_status[r];
+            const uint32_t missing = __ballot_sync(0xffffffffu, st == 0), ends = __ballot_sync(0xffffffffu, (st & kScanPrefix) != 0);
+            // lanes before the first range that is not there yet, up to the first prefix
+            const uint32_t known = missing ? (missing & (0u - missing)) - 1u : 0xffffffffu;
+            const uint32_t end = ends & known;
+            if (!end && missing)
             {
-                unsigned long long st = 0;
-                int spins = 0;
-                do
-                    st = *(volatile unsigned long long*)&a.scan_status[j];
-                while (st == 0 && ++spins < spin_limit);
-                if (st == 0)
+                if (++spins >= spin_limit)
                 {
                     // a range never published: report it, never hang
-                    atomicOr(&a.status->error, 3u);  // EDXR_ERR_TIMEOUT
+                    if (lane == 0)
+                        atomicOr(&a.status->error, 3u);  // EDXR_ERR_TIMEOUT
                     break;
                 }
-                prefix += (uint32_t)st;
-                if (st & kScanPrefix)
-                    break;
-                j--;
+                continue;
             }
-            if (publish)
-                atomicExch(&a.scan_status[b], kScanPrefix | (prefix + total));
+            const uint32_t take = end ? (end ^ (end - 1u)) : 0xffffffffu;  // up to the first prefix
+            prefix += __reduce_add_sync(0xffffffffu, (take >> lane) & 1u ? (uint32_t)st : 0u);
+            if (end)
+                break;
+            j -= 32;
+            spins = 0;
         }
-        s_prefix = prefix;
+        if (publish)
+            atomicExch(&a.scan_status[b], kScanPrefix | (prefix + total));
+        if (lane == 0)
+            s_prefix = prefix;
     }
     __syncthreads();
     const uint32_t prefix = s_prefix;
@@ -1114,9 +1136,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
     // did not all fit (the unsorted list or the bins overflowed) is rendered
     // again by the host; its tiles are made empty here, so no raster item
     // reads a bin with missing entries or leaves a split tile's keys behind.
-    const bool dropped =
-        __syncthreads_or(threadIdx.x < (uint32_t)kBinStripes &&
-                         *(volatile uint32_t*)stripe_counter(a, threadIdx.x) > stripe_slots(a.bin_capacity)) != 0;
+    const bool dropped = s_dropped;
     // entries per work item; items of at least 3/4 of that are heavy
     const uint32_t E = (uint32_t)a.tune.item_entries, heavy_min = E - E / 4;
     uint32_t run = prefix + incl - sum;
@@ -1147,7 +1167,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
     }
     // one atomic per warp and list (light and empty counts, at most 128 each,
     // share a word)
-    const uint32_t lane = threadIdx.x & 31;
     const uint32_t packed = nlight | (nempty << 16);
     uint32_t hincl = nheavy, pincl = packed;
 #pragma unroll
@@ -1201,19 +1220,20 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
     }
 
     // the range holding the last tile has the grand total
-    if (a.total_tiles > 0 && b == (a.total_tiles - 1) / kScanBlock && threadIdx.x == kScanThreads - 1)
+    if (a.total_tiles > 0 && b == (a.total_tiles - 1) / kScanBlock && threadIdx.x >= kScanThreads - 32)
     {
         const uint64_t grand = prefix + total;
-        a.tile_offset[a.total_tiles] = (uint32_t)grand;
         // the unsorted list's stripes share the capacity: the fullest decides
-        uint64_t fullest = 0, entries = 0, survivors = 0;
-        for (int r = 0; r < kBinStripes; r++)
+        const uint64_t fullest = __reduce_max_sync(0xffffffffu, filled);
+        uint64_t entries = filled, survivors = survived;
+        for (int o = 16; o >= 1; o >>= 1)
         {
-            const uint32_t* c = stripe_counter(a, (uint32_t)r);
-            fullest = max(fullest, (uint64_t)c[0]);
-            entries += c[0];
-            survivors += c[1];
+            entries += __shfl_down_sync(0xffffffffu, entries, o);
+            survivors += __shfl_down_sync(0xffffffffu, survivors, o);
         }
+        if (lane != 0)
+            return;
+        a.tile_offset[a.total_tiles] = (uint32_t)grand;
         const uint64_t needed = max(grand, fullest * kBinStripes);
         a.status->bins_needed = needed;
         a.status->bin_entries = entries;
