@@ -885,8 +885,14 @@ __global__ void __launch_bounds__(256, 4) k_bin_big(PassArgs a)
     };
     // batches of up to 32 triangles, small enough that every warp gets one
     const uint32_t batch = min(32u, max(1u, (nb + nw - 1) / nw));
+    // with few triangles, several warps share one, each taking every parts-th
+    // 32 of its tiles (a triangle over the whole screen is 7 rounds for one
+    // warp at 1366x769, 255 at 3840x2160)
+    const uint32_t parts = nb ? min(32u, max(1u, nw / nb)) : 1u;
+    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int part = (int)(gw % parts);
     const bool early_cull = nb >= a.total_tiles;
-    for (uint32_t b0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * batch; b0 < nb; b0 += nw * batch)
+    for (uint32_t b0 = gw / parts * batch; b0 < nb; b0 += max(1u, nw / parts) * batch)
     {
         // this lane's triangle of the batch and its number of 32x32 tiles
         uint32_t mine = kNoTriangle, mine_zocc = 0xFFFFFFFFu;
@@ -907,7 +913,7 @@ __global__ void __launch_bounds__(256, 4) k_bin_big(PassArgs a)
             if (lane >= (uint32_t)o) incl += v;
         }
         const int pairs = __shfl_sync(0xffffffffu, incl, 31);
-        for (int base = 0; base < pairs; base += 32)
+        for (int base = 32 * part; base < pairs; base += 32 * (int)parts)
         {
             const int p = base + (int)lane;
             // owner: the first lane whose inclusive count exceeds p
@@ -2654,13 +2660,16 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
     if (a.total_tris)
     {
         go(k_setup, (a.total_tris + 255) / 256, 256, 0);
-        go(k_clip, sms * 8, kClipThreads, 0);
+        // (no more blocks than one 16-lane group per triangle fills)
+        go(k_clip, min((uint32_t)sms * 8u, (a.total_tris + 7u) / 8u), kClipThreads, 0);
     }
     go(k_bin_big, sms * 4, 256, 0);
     mark(2);
     go(k_scan, nscan, kScanThreads, 0);
     mark(3);
-    go(k_bin_move, sms * (a.tune.bin_blocks_per_sm > 0 ? a.tune.bin_blocks_per_sm : 8), 256, 0);
+    // (two blocks per SM at least, more by about two entries per triangle)
+    const uint32_t move = (uint32_t)sms * (uint32_t)(a.tune.bin_blocks_per_sm > 0 ? a.tune.bin_blocks_per_sm : 8);
+    go(k_bin_move, min(move, max((uint32_t)sms * 2u, a.total_tris / 128u)), 256, 0);
     mark(4);
     if (a.msaa_log2 > 0)
     {
