@@ -1622,19 +1622,8 @@ __device__ __forceinline__ void group_sync(int group)
     }
 }
 
-// Merges key k into a shared key: other warps of the group may write the same
-// one (Group > 1), or only this lane does.
-template <int Group>
-__device__ __forceinline__ void lower_key(unsigned long long* slot, unsigned long long k)
-{
-    if (Group == 1)
-        *slot = k;
-    else
-        atomicMin(slot, k);
-}
-
-// Group warps share an item (1: a warp per item; 2, 4 or 8 where the frame
-// has too few tiles to give every warp one, see raster_group).
+// Group warps share an item (1: a warp per item; 4 or 8 where the frame has
+// too few tiles to give every warp one, see raster_group).
 // 3 blocks per SM: the 80 registers a thread hold the shading without spills.
 // At 5 blocks (48 registers, 156 bytes spilled) the raster stage took 119
 // instead of 100 us on the terrain (2,097,152 triangles, 1920x1080), 235
@@ -1650,7 +1639,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
     constexpr int kPixels = 256 / kThreads;         // pixels of the tile per thread
     __shared__ unsigned long long s_key[kGroups][256];
     __shared__ StagedSlot s_tri[kRasterWarps][32];
-    __shared__ uint32_t s_next[kGroups], s_done[kGroups];
+    __shared__ uint32_t s_next[kGroups], s_done[kGroups], s_staged[kRasterWarps], s_bound[kRasterWarps];
     report_status(a);
     if (*(volatile uint32_t*)&a.status->error)
         return;  // the pass failed (see k_bin_move); every thread of the block leaves
@@ -1778,9 +1767,9 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
         uint32_t tzmax = tzocc;
 
         // each chunk's bin entries load while the previous chunk is rasterized
-        for (uint32_t c = c0; c < e1; c += kThreads)
+        for (uint32_t c = c0, cg = e0; cg < e1; c += kThreads, cg += kThreads)
         {
-            const uint32_t m = min(32u, e1 - c);
+            const uint32_t m = c < e1 ? min(32u, e1 - c) : 0u;
             const uint32_t entry = next;
             if (c + kThreads + lane < e1)
                 next = a.bins[c + kThreads + lane];
@@ -1852,9 +1841,9 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                 }
             }
             __syncwarp();
-            // Other entries: the whole warp over each region in turn, in
-            // blocks of 16, 8 or 4 columns and two rows of blocks at a time.
-            for (int j = nsm; j < nst; j++)
+            // Other entries, a warp alone: the whole warp over each region in
+            // turn.
+            for (int j = nsm; Group == 1 && j < nst; j++)
             {
                 const StagedTri s = staged[j].s;
                 const uint32_t fl = s.flags;
@@ -1871,14 +1860,66 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                     const bool hit = fragment_key(s, x, y, less, k);
                     const unsigned long long cur = key[y * 16 + x];
                     if (hit && k < cur)
-                        lower_key<Group>(&key[y * 16 + x], k);
+                        key[y * 16 + x] = k;
                 }
                 __syncwarp();
             }
-            if (c + kThreads < e1)
+            // Several warps: each thread over its own pixels (the ones it
+            // shades) and every warp's staged entries, so no key is shared and
+            // none needs an atomic.
+            if (Group > 1)
             {
-                // (keys only fall, so a bound from keys that other warps are
-                // still lowering is a valid, larger one)
+                if (lane == 0)
+                    s_staged[warp] = (uint32_t)nsm | ((uint32_t)nst << 8);
+                group_sync<Group>(group);  // every warp's entries staged, its small ones rasterized
+                unsigned long long mine[kPixels];
+                const int x = gthread & 15, row = gthread >> 4;
+#pragma unroll
+                for (int k = 0; k < kPixels; k++)
+                    mine[k] = key[gthread + kThreads * k];
+                for (int w = 0; w < Group; w++)
+                {
+                    const uint32_t range = s_staged[group * Group + w];
+                    for (uint32_t j = range & 255u; j < range >> 8; j++)
+                    {
+                        const StagedTri& t = s_tri[group * Group + w][j].s;
+                        const uint32_t fl = t.flags;
+                        const int rx0 = fl & 31, rx1 = (fl >> 5) & 31, ry0 = (fl >> 10) & 31, ry1 = (fl >> 15) & 31;
+#pragma unroll
+                        for (int k = 0; k < kPixels; k++)
+                        {
+                            const int y0 = 2 * (int)gwarp + (kThreads >> 4) * k;  // the warp's two rows
+                            if (y0 + 1 < ry0 || y0 > ry1)
+                                continue;
+                            const int y = row + (kThreads >> 4) * k;
+                            uint64_t kk;
+                            const bool hit = fragment_key(t, x, y, less, kk);
+                            if (hit && x >= rx0 && x <= rx1 && y >= ry0 && y <= ry1 && kk < mine[k])
+                                mine[k] = kk;
+                        }
+                    }
+                }
+                uint32_t mz = 0;
+#pragma unroll
+                for (int k = 0; k < kPixels; k++)
+                {
+                    key[gthread + kThreads * k] = mine[k];
+                    mz = max(mz, (uint32_t)(mine[k] >> 32));
+                }
+                mz = __reduce_max_sync(0xffffffffu, mz);
+                if (lane == 0)
+                    s_bound[warp] = mz;
+                group_sync<Group>(group);  // before the entries are staged over
+                if (cg + kThreads < e1)
+                {
+                    uint32_t b = 0;
+                    for (int w = 0; w < Group; w++)
+                        b = max(b, s_bound[group * Group + w]);
+                    tzmax = min(tzocc, b);
+                }
+            }
+            else if (c + kThreads < e1)
+            {
                 uint32_t mz = 0;
 #pragma unroll
                 for (int k = 0; k < 8; k++)
@@ -1886,8 +1927,6 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                 tzmax = min(tzocc, __reduce_max_sync(0xffffffffu, mz));
             }
         }
-        if (Group > 1)
-            group_sync<Group>(group);
 
         // A tile split into several items merges its keys in the key buffer;
         // the item that finishes last (the one whose entries bring the tile's
@@ -2553,23 +2592,30 @@ static cudaError_t launch_raster(int sms, const PassArgs& a, cudaStream_t s, boo
 // Warps per raster item.  A warp alone takes 10 to 25 us for a tile (a chain
 // of dependent loads, then eight rounds of shading), so a frame with fewer
 // tiles than resident warps (24 per SM) leaves most of the chip idle for that
-// long; more warps per tile shorten it.  Against it stand the barriers and,
-// with more than one warp, a 64-bit shared atomic per pixel of a large region
-// instead of a store, so frames of few triangles per tile (large regions) and
-// frames with several tiles per warp keep one.  Raster stage, 1 / 2 / 4 / 8
-// warps, us: sphere (4,032 triangles) 320x180, 240 tiles, 27.6 / 20.1 / 18.4 /
-// 16.4; 128x128-quad terrain 640x400, 1,000 tiles, 42.3 / 33.8 / 32.4 / 30.4;
-// 200x200 quads 800x520, 1,650 tiles, 47.1 / 36.5 / 35.8 / 36.2; 256x256 quads
-// 1280x720, 3,600 tiles, textured, 76 / 67; 301x301 quads 1366x769, 4,214
-// tiles, 56 / 53; sphere 1280x720 (1.1 triangles per tile) 24.6 / 28.7;
-// 2,097,152-triangle terrain, 8,160 tiles, 96 / 99; binning stress, 32,400
-// tiles, 215 / 310.
+// long; more warps per tile shorten it.  Against it stand the barriers and that
+// every warp looks at every large region, so frames with several tiles per
+// warp keep one.  Raster stage with 1 / 2 / 4 / 8 warps, us:
+//   sphere (4,032 triangles) 320x180, 240 tiles      28.0 / 18.4 / 16.4 / 16.0
+//   96x96-quad terrain 480x270, 510 tiles            42.0 / 30.7 / 23.6 / 20.5
+//   10,000 stress triangles 480x270                  56.3 / 46.1 / 31.8 / 33.1
+//   128x128-quad terrain 640x400, 1,000 tiles        41.0 / 30.4 / 25.6 / 23.6
+//   sphere 1280x720, 3,600 tiles                     23.6 / 24.2 / 19.1 / 20.1
+//   256x256-quad terrain 1280x720, textured          69.3 / 61.1 / 56.3 / 63.5
+//   301x301-quad terrain 1366x769, 4,214 tiles       53.6 / 46.8 / 45.1 / 56.0
+//   100,000 stress triangles 1600x900, 5,700 tiles   64.2 / 71.7 / 73.7 / 96.6
+//   512x512-quad terrain 1760x990, 6,820 tiles       67.9 / 68.6 / 69.3 / 87.1
+//   sphere (16,256 triangles) 1920x1080, 8,160 tiles 31.1 / 26.6 / 26.6 / 32.8
+//   terrain (2,097,152 triangles) 1920x1080          93.9 / 102  / 103  / 123
+// Two warps are best nowhere; above 30 tiles per SM four pay only where the
+// triangles are few, so that most tiles have a handful of large regions or none.
 static int raster_group(const PassArgs& a, int sms)
 {
-    const uint64_t tiles = a.total_tiles, warps = 24ull * (uint64_t)sms;
-    if (a.tune.raster_variant == 0 || a.total_tris < 8 * tiles)
+    const uint64_t tiles = a.total_tiles, n = (uint64_t)sms;
+    if (a.tune.raster_variant == 0)
         return 1;
-    return 8 * tiles <= warps + warps / 8 ? 8 : 2 * tiles <= warps ? 4 : tiles <= warps + warps / 4 ? 2 : 1;
+    if (8 * tiles <= 27 * n)
+        return 8;
+    return tiles <= 30 * n || (tiles <= 60 * n && a.total_tris <= 120 * n) ? 4 : 1;
 }
 
 // Resident blocks per SM of k_raster_ms with 2^level samples (the dynamic
@@ -2607,7 +2653,6 @@ static int ms_occupancy(int level)
 void prepare_kernels()
 {
     raster_occupancy<1>();
-    raster_occupancy<2>();
     raster_occupancy<4>();
     raster_occupancy<8>();
     for (int level = 1; level <= kMaxMsaaLog2; level++)
@@ -2693,7 +2738,6 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
         {
         case 8: e = launch_raster<8>(sms, a, s, follows); break;
         case 4: e = launch_raster<4>(sms, a, s, follows); break;
-        case 2: e = launch_raster<2>(sms, a, s, follows); break;
         default: e = launch_raster<1>(sms, a, s, follows); break;
         }
     }
