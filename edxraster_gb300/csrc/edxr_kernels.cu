@@ -324,42 +324,44 @@ __global__ void __launch_bounds__(256, 6) k_setup(PassArgs a)
             straddle = (k0 | k1 | k2) != 0 && !(k0 & k1 & k2);
         }
     }
-    // warp-wide exclusive scans of the queued triangles and of the bin
-    // entries; one atomic per warp on the clip queue (few warps have any)
-    // and on the warp's stripe of the unsorted list
-    uint32_t qincl = straddle ? 1u : 0u, eincl = nent;
+    // A warp whose triangles are all culled has nothing to append: half the
+    // warps of a frame whose mesh reaches beyond the view or turns away.
+    const uint32_t kept = __ballot_sync(0xffffffffu, nOut != 0), queued = __ballot_sync(0xffffffffu, straddle);
+    if (!(kept | queued))
+        return;
+    // places of the queued triangles and of the bin entries within the warp
+    // (an entry count has five bits: at most 16 tiles), one atomic per warp on
+    // the clip queue (few warps have any) and on the warp's stripe of the
+    // unsorted list
+    const uint32_t before = (1u << lane) - 1u;
+    uint32_t eexcl = 0, etotal = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
+    for (int o = 0; o < 5; o++)
     {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, qincl, o);
-        const uint32_t ve = __shfl_up_sync(0xffffffffu, eincl, o);
-        if (lane >= (uint32_t)o)
-        {
-            qincl += v;
-            eincl += ve;
-        }
+        const uint32_t bit = __ballot_sync(0xffffffffu, (nent >> o) & 1u);
+        eexcl += (uint32_t)__popc(bit & before) << o;
+        etotal += (uint32_t)__popc(bit) << o;
     }
     const uint32_t stripe = warp_stripe();
-    const uint32_t survivors = __popc(__ballot_sync(0xffffffffu, nOut != 0));
     uint32_t qbase = 0, ebase = 0;
-    if (lane == 31)
+    if (lane == 0)
     {
-        if (survivors)
-            atomicAdd(stripe_counter(a, stripe) + 1, survivors);  // statistics
-        qbase = qincl ? atomicAdd(&a.counters[4], qincl) : 0u;
-        ebase = eincl ? atomicAdd(stripe_counter(a, stripe), eincl) : 0u;
+        if (kept)
+            atomicAdd(stripe_counter(a, stripe) + 1, (uint32_t)__popc(kept));  // statistics
+        qbase = queued ? atomicAdd(&a.counters[4], (uint32_t)__popc(queued)) : 0u;
+        ebase = etotal ? atomicAdd(stripe_counter(a, stripe), etotal) : 0u;
     }
-    qbase = __shfl_sync(0xffffffffu, qbase, 31);
-    ebase = __shfl_sync(0xffffffffu, ebase, 31);
-    if (straddle)
+    ebase = __shfl_sync(0xffffffffu, ebase, 0);
+    if (queued)
     {
-        const uint32_t q = qbase + qincl - 1u;
-        if (q < a.poly_capacity)
+        qbase = __shfl_sync(0xffffffffu, qbase, 0);
+        const uint32_t q = qbase + (uint32_t)__popc(queued & before);
+        if (straddle && q < a.poly_capacity)
             a.clip_list[q] = gi;
     }
     // an unclipped triangle's record sits at its flattened index
     const uint64_t sbegin = stripe_begin(a, stripe);
-    const uint64_t slot = sbegin + ebase + eincl - nent;
+    const uint64_t slot = sbegin + ebase + eexcl;
     if (nOut)
     {
         t.order = tri << 4;
