@@ -1472,6 +1472,42 @@ struct PixelOut
     uint32_t* tri_id;
 };
 
+// The per-vertex-attribute shaders (Blinn-Phong, Lambertian with or without
+// albedo) at barycentrics (L0, L1) of raster triangle t: perspective-correct
+// weights, the vertices' attributes, the shading model.  No call inside.
+template <bool Full>
+static __device__ __forceinline__ float3 shade_common(const FrameDesc& f, const RTri& t, const ClipPoly* polys,
+                                                      float L0, float L1)
+{
+    float b0 = L0, b1 = L1;
+    float b2 = fsub(fsub(1.0f, b0), b1);
+    b0 = fmul(b0, t.invW0);
+    b1 = fmul(b1, t.invW1);
+    b2 = fmul(b2, t.invW2);
+    const float invB = __frcp_rn(fadd(fadd(b0, b1), b2));
+    b0 = fmul(b0, invB);
+    b1 = fmul(b1, invB);
+    b2 = fsub(fsub(1.0f, b0), b1);
+    const ShadeVerts v = shade_verts<false, Full>(f, t, polys);
+    return shade_model(f, lerp3(b0, v.p[0], b1, v.p[1], b2, v.p[2]), lerp3(b0, v.n[0], b1, v.n[1], b2, v.n[2]),
+                       lerp3(b0, v.a[0], b1, v.a[1], b2, v.a[2]));
+}
+
+// Is the frame shaded out of line (the reference Blinn-Phong and the textured
+// shaders, and meshes without normals or albedo)?
+__device__ __forceinline__ bool slow_shading(const FrameDesc& f)
+{
+    return f.ps_kind == 1 || f.ps_kind == 4 || !full_mesh(f);
+}
+
+static __device__ __forceinline__ float3 shade_slow(const FrameDesc& f, const RTri& t, const RTri* tg,
+                                                    const ClipPoly* polys, float L0, float L1, int px, int py)
+{
+    if (f.ps_kind == 1 || f.ps_kind == 4)
+        return shade_fragment(f, t, tg, polys, L0, L1, px, py);
+    return shade_common<false>(f, t, polys, L0, L1);
+}
+
 static __device__ __forceinline__ void write_pixel(const PixelOut a, const FrameDesc& f, uint32_t ri, uint64_t pix, int px,
                                                 int py)
 {
@@ -1491,30 +1527,10 @@ static __device__ __forceinline__ void write_pixel(const PixelOut a, const Frame
     const float L1 = fmul(__int2float_rn(n2), t.invDet);
     const float L2 = fsub(fsub(1.0f, L0), L1);
     const float d = fadd(fadd(fmul(L0, t.z0), fmul(L1, t.z1)), fmul(L2, t.z2));
-    const float3 c = shade_fragment(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
+    const float3 c = shade_slow(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
     a.color[pix] = make_float4(c.x, c.y, c.z, 1.0f);
     a.depth[pix] = d;
     a.tri_id[pix] = t.order >> 4;
-}
-
-// The per-vertex-attribute shaders (Blinn-Phong, Lambertian with or without
-// albedo) at barycentrics (L0, L1) of raster triangle t: perspective-correct
-// weights, the vertices' attributes, the shading model.  No call inside.
-static __device__ __forceinline__ float3 shade_common(const FrameDesc& f, const RTri& t, const ClipPoly* polys,
-                                                      float L0, float L1)
-{
-    float b0 = L0, b1 = L1;
-    float b2 = fsub(fsub(1.0f, b0), b1);
-    b0 = fmul(b0, t.invW0);
-    b1 = fmul(b1, t.invW1);
-    b2 = fmul(b2, t.invW2);
-    const float invB = __frcp_rn(fadd(fadd(b0, b1), b2));
-    b0 = fmul(b0, invB);
-    b1 = fmul(b1, invB);
-    b2 = fsub(fsub(1.0f, b0), b1);
-    const ShadeVerts v = shade_verts(f, t, polys);
-    return shade_model(f, lerp3(b0, v.p[0], b1, v.p[1], b2, v.p[2]), lerp3(b0, v.n[0], b1, v.n[1], b2, v.n[2]),
-                       lerp3(b0, v.a[0], b1, v.a[1], b2, v.a[2]));
 }
 
 // The one write of a pixel for the per-vertex-attribute shaders: no call
@@ -1532,7 +1548,7 @@ static __device__ __forceinline__ void write_pixel_fast(const PixelOut a, const 
     const RTri t = a.rtris[ri];
     float L0, L1;
     const float d = depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
-    const float3 c = shade_common(f, t, a.polys, L0, L1);
+    const float3 c = shade_common<true>(f, t, a.polys, L0, L1);
     a.color[pix] = make_float4(c.x, c.y, c.z, 1.0f);
     a.depth[pix] = d;
     a.tri_id[pix] = t.order >> 4;
@@ -1983,7 +1999,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                 }
             }
         }
-        if (shade && (f.ps_kind == 1 || f.ps_kind == 4))
+        if (shade && slow_shading(f))
             shade_tile_slow(out, f, key, gthread, kThreads, tileX, tileY, less, nr, a.tri_first, a.total_tris);
         else if (shade)
         {
@@ -2120,8 +2136,8 @@ static __device__ __forceinline__ void write_pixel_ms(const PassArgs& a, const F
             id = t.order >> 4;
             float L0, L1;
             depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
-            const float3 c = Common ? shade_common(f, t, a.polys, L0, L1)
-                                    : shade_fragment(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
+            const float3 c = Common ? shade_common<true>(f, t, a.polys, L0, L1)
+                                    : shade_slow(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
             rgb = to_byte(c.x) | (to_byte(c.y) << 8) | (to_byte(c.z) << 16);
         }
 #pragma unroll (S <= 8 ? S : 4)
@@ -2511,7 +2527,7 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
                 __syncthreads();
             }
         }
-        if (shade && (f.ps_kind == 1 || f.ps_kind == 4))
+        if (shade && slow_shading(f))
             shade_tile_ms_slow<S>(a, f, key, (int)threadIdx.x, kThreads, tileX, tileY, less, nr);
         else if (shade)
         {
