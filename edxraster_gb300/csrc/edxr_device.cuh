@@ -483,12 +483,11 @@ struct ShadeVerts
 // nine loads for a missing array was some 40 of its 350 instructions (raster
 // stage: binning stress 210 -> 202 us, terrain at 4 samples 238 -> 229).
 template <bool NormalsOnly = false, bool Full = false>
-__device__ __forceinline__ ShadeVerts shade_verts(const FrameDesc& f, const RTri& t, const ClipPoly* polys)
+__device__ __forceinline__ ShadeVerts shade_verts(const FrameDesc& f, const RTri& t, const ClipPoly* polys,
+                                                  const uint32_t* vi = nullptr)
 {
-    const uint32_t tri = t.order >> 4;
-    const uint32_t i0 = __ldg(f.indices + 3 * (size_t)tri + 0);
-    const uint32_t i1 = __ldg(f.indices + 3 * (size_t)tri + 1);
-    const uint32_t i2 = __ldg(f.indices + 3 * (size_t)tri + 2);
+    const uint32_t* idx = vi ? vi : f.indices + 3 * (size_t)(t.order >> 4);
+    const uint32_t i0 = vi ? vi[0] : __ldg(idx), i1 = vi ? vi[1] : __ldg(idx + 1), i2 = vi ? vi[2] : __ldg(idx + 2);
     const char* pos = NormalsOnly ? nullptr : f.positions;
     const char* alb = NormalsOnly ? nullptr : f.albedo;
     float3 sp[3] = { ld3<Full>(pos, f.pos_stride, i0, 0.f), ld3<Full>(pos, f.pos_stride, i1, 0.f), ld3<Full>(pos, f.pos_stride, i2, 0.f) };

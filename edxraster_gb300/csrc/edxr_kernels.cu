@@ -1477,7 +1477,7 @@ struct PixelOut
 // weights, the vertices' attributes, the shading model.  No call inside.
 template <bool Full>
 static __device__ __forceinline__ float3 shade_common(const FrameDesc& f, const RTri& t, const ClipPoly* polys,
-                                                      float L0, float L1)
+                                                      float L0, float L1, const uint32_t* vi = nullptr)
 {
     float b0 = L0, b1 = L1;
     float b2 = fsub(fsub(1.0f, b0), b1);
@@ -1488,7 +1488,7 @@ static __device__ __forceinline__ float3 shade_common(const FrameDesc& f, const 
     b0 = fmul(b0, invB);
     b1 = fmul(b1, invB);
     b2 = fsub(fsub(1.0f, b0), b1);
-    const ShadeVerts v = shade_verts<false, Full>(f, t, polys);
+    const ShadeVerts v = shade_verts<false, Full>(f, t, polys, vi);
     return shade_model(f, lerp3(b0, v.p[0], b1, v.p[1], b2, v.p[2]), lerp3(b0, v.n[0], b1, v.n[1], b2, v.n[2]),
                        lerp3(b0, v.a[0], b1, v.a[1], b2, v.a[2]));
 }
@@ -1536,7 +1536,7 @@ static __device__ __forceinline__ void write_pixel(const PixelOut a, const Frame
 // The one write of a pixel for the per-vertex-attribute shaders: no call
 // inside.
 static __device__ __forceinline__ void write_pixel_fast(const PixelOut a, const FrameDesc& f, uint32_t ri,
-                                                        uint64_t pix, int px, int py)
+                                                        uint64_t pix, int px, int py, uint32_t rank)
 {
     if (ri == kNoTriangle)
     {
@@ -1545,13 +1545,17 @@ static __device__ __forceinline__ void write_pixel_fast(const PixelOut a, const 
         a.tri_id[pix] = kNoTriangle;
         return;
     }
+    // the rank names the input triangle: its indices load beside its record
+    const uint32_t tri = ((rank - 1u) >> 4) - f.tri_base;
+    const uint32_t* idx = f.indices + 3 * (size_t)tri;
+    const uint32_t vi[3] = { __ldg(idx), __ldg(idx + 1), __ldg(idx + 2) };
     const RTri t = a.rtris[ri];
     float L0, L1;
     const float d = depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
-    const float3 c = shade_common<true>(f, t, a.polys, L0, L1);
+    const float3 c = shade_common<true>(f, t, a.polys, L0, L1, vi);
     a.color[pix] = make_float4(c.x, c.y, c.z, 1.0f);
     a.depth[pix] = d;
-    a.tri_id[pix] = t.order >> 4;
+    a.tri_id[pix] = tri;
 }
 
 // A tile shaded by the FP64 or the textured shader: out of line, pixel by
@@ -2009,9 +2013,11 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
                 const int p = gthread + kThreads * k;
                 const int px = (tileX << 4) + (p & 15), py = (tileY << 4) + (p >> 4);
                 const uint32_t low = (uint32_t)key[p];
-                const uint32_t ri = raster_triangle_of(a, less ? low : ~low, nr);
+                const uint32_t rank = less ? low : ~low;
+                const uint32_t ri = raster_triangle_of(a, rank, nr);
                 if (px < f.width && py < f.height)
-                    write_pixel_fast(out, f, ri, f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px, px, py);
+                    write_pixel_fast(out, f, ri, f.pix_base + (uint64_t)py * (uint32_t)f.width + (uint32_t)px, px, py,
+                                     rank);
             }
         }
         group_sync<Group>(group);
