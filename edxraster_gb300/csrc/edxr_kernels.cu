@@ -2706,7 +2706,16 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
     if (a.msaa_log2 > 0)
         a.tune.item_entries = min(1024, a.tune.item_entries * (a.msaa_log2 <= 3 ? 2 : 4));
     else
-        a.tune.item_entries = min(1024, a.tune.item_entries * raster_group(a, sms));
+    {
+        // Several warps share an item; and with many small frames, four tiles
+        // and more per warp, the last items are a small part of the pass, so
+        // fewer tiles need splitting (raster stage, 128 / 256 entries: 256
+        // views at 512x512 722 / 709 us, 64 views of a torus at 256x256 122 /
+        // 113, 90 views at 300x200 96 / 92; 12 views there 25 / 30; the frames
+        // of one mesh, terrain 92 / 103, binning stress 200 / 203).
+        const bool many = a.num_frames > 1 && (uint64_t)a.total_tiles >= 96ull * (uint64_t)sms;
+        a.tune.item_entries = min(1024, a.tune.item_entries * (many ? 2 : raster_group(a, sms)));
+    }
     const uint32_t nscan = scan_blocks(a.total_tiles);
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
