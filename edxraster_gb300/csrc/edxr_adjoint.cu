@@ -34,28 +34,6 @@ constexpr int kWarps = 4;
 constexpr int kThreads = 32 * kWarps;
 constexpr int kSpan = 256;
 
-// Frame of flattened output pixel p: one division when the pass's frames
-// share one resolution (tiles_per_frame set: the batched pass), else a
-// search over the frames' first pixels.
-__device__ __forceinline__ uint32_t frame_of_pixel(const PassArgs& a, uint64_t p)
-{
-    if (a.tiles_per_frame)
-    {
-        const uint64_t per_frame = a.total_pixels / a.num_frames;
-        return a.total_pixels <= 0xFFFFFFFFull ? (uint32_t)p / (uint32_t)per_frame : (uint32_t)(p / per_frame);
-    }
-    const FrameDesc* frames = a.frames;
-    const uint32_t n = a.num_frames;
-    uint32_t lo = 0, hi = n - 1;
-    while (lo < hi)
-    {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (frames[mid].pix_base <= p) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
 struct V3
 {
     float x, y, z;
@@ -65,7 +43,14 @@ __device__ __forceinline__ V3 operator+(V3 a, V3 b) { return { a.x + b.x, a.y + 
 __device__ __forceinline__ V3 operator-(V3 a, V3 b) { return { a.x - b.x, a.y - b.y, a.z - b.z }; }
 __device__ __forceinline__ V3 operator*(float s, V3 a) { return { s * a.x, s * a.y, s * a.z }; }
 __device__ __forceinline__ float dot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ float len(V3 a) { return sqrtf(dot(a, a)); }
+// 1 / |a|: the hardware estimate and one Newton step on its residual; an
+// estimate that is not finite (a zero or overflowing square) stays as it is.
+__device__ __forceinline__ float inv_len(V3 a)
+{
+    const float x = dot(a, a), y = rsqrtf(x);
+    const float e = x > 0.0f && x < 3.0e38f ? fmaf(-(x * y), y, 1.0f) : 0.0f;
+    return fmaf(0.5f * y, e, y);
+}
 __device__ __forceinline__ V3 ld(const char* base, uint32_t stride, uint32_t i, float dflt)
 {
     if (!base)
@@ -73,8 +58,8 @@ __device__ __forceinline__ V3 ld(const char* base, uint32_t stride, uint32_t i, 
     const float* p = reinterpret_cast<const float*>(base + (size_t)i * stride);
     return v3(__ldg(p), __ldg(p + 1), __ldg(p + 2));
 }
-// gradient of normalize(x) applied to dy: (dy - y (y . dy)) / |x|
-__device__ __forceinline__ V3 normalize_grad(V3 y, float lenx, V3 dy) { return (1.0f / lenx) * (dy - dot(y, dy) * y); }
+// gradient of y = normalize(x) applied to dy: (dy - y (y . dy)) / |x|
+__device__ __forceinline__ V3 normalize_grad(V3 y, float invx, V3 dy) { return invx * (dy - dot(y, dy) * y); }
 
 // m0 x + m1 y + m2 z + m3 as a pair.
 __device__ __forceinline__ FF ff_dot4(float m0, float m1, float m2, float m3, float x, float y, float z)
@@ -168,21 +153,21 @@ __device__ __forceinline__ bool pixel_forward(const FrameDesc& f, const DiffMesh
 struct ShadeTerms
 {
     V3 Nn, L, E, H;
-    float nlen, llen, elen, hlen;
+    float ninv, einv, hinv;  // 1 / length before normalisation
     float nl, nh, nhc, powv, diffuse, spec;
     bool albedo, specular, clamp;
 };
 
-// Light, ks and shininess in effect for frame f.
+// Light (normalised, and 1 / its length), ks and shininess in effect for frame f.
 struct Shading
 {
-    float light[3], ks, shininess;
+    float light[3], light_inv, ks, shininess;
 };
 __device__ __forceinline__ Shading shading_of(const FrameDesc& f, const DiffMesh& m)
 {
     if (m.override_shading)
-        return { { m.light[0], m.light[1], m.light[2] }, m.ks, m.shininess };
-    return { { f.light_raw[0], f.light_raw[1], f.light_raw[2] }, f.ks, f.shininess };
+        return { { m.light[0], m.light[1], m.light[2] }, m.light_inv, m.ks, m.shininess };
+    return { { f.light[0], f.light[1], f.light[2] }, f.light_inv, f.ks, f.shininess };
 }
 
 __device__ __forceinline__ V3 shade_forward(const FrameDesc& f, const Shading& sh, const PixelState& s,
@@ -191,22 +176,20 @@ __device__ __forceinline__ V3 shade_forward(const FrameDesc& f, const Shading& s
     t.albedo = (f.ps_kind == 0 || f.ps_kind == 2);
     t.specular = (f.ps_kind <= 1);
     t.clamp = (f.ps_kind == 0);
-    t.nlen = len(s.Nraw);
-    t.Nn = (1.0f / t.nlen) * s.Nraw;
-    const V3 l = v3(sh.light[0], sh.light[1], sh.light[2]);
-    t.llen = len(l);
-    t.L = (1.0f / t.llen) * l;
+    t.ninv = inv_len(s.Nraw);
+    t.Nn = t.ninv * s.Nraw;
+    t.L = v3(sh.light[0], sh.light[1], sh.light[2]);
     t.nl = dot(t.L, t.Nn);
     t.diffuse = (fmaxf(t.nl, 0.0f) + 0.2f) * 0.954929658551372f;
     t.spec = 0.0f;
     if (t.specular)
     {
         const V3 Er = v3(f.eye[0], f.eye[1], f.eye[2]) - s.P;
-        t.elen = len(Er);
-        t.E = (1.0f / t.elen) * Er;
+        t.einv = inv_len(Er);
+        t.E = t.einv * Er;
         const V3 Hr = t.L + t.E;
-        t.hlen = len(Hr);
-        t.H = (1.0f / t.hlen) * Hr;
+        t.hinv = inv_len(Hr);
+        t.H = t.hinv * Hr;
         t.nh = dot(t.Nn, t.H);
         t.nhc = t.clamp ? fmaxf(t.nh, 0.0f) : t.nh;
         t.powv = powf(t.nhc, sh.shininess);
@@ -215,6 +198,34 @@ __device__ __forceinline__ V3 shade_forward(const FrameDesc& f, const Shading& s
     if (t.albedo)
         return v3(s.A.x * t.diffuse + t.spec, s.A.y * t.diffuse + t.spec, s.A.z * t.diffuse + t.spec);
     return v3(t.diffuse + t.spec, t.diffuse + t.spec, t.diffuse + t.spec);
+}
+
+// Where a span's pixels lie: the frame of its first pixel and that pixel's
+// place in it.  The frames of a pass have one size, so this is one 64-bit
+// division per warp; a pixel's row is a 32-bit one.
+struct Span
+{
+    uint32_t frame, offset;
+};
+__device__ __forceinline__ Span span_of(uint64_t base, uint32_t frame_pixels)
+{
+    const uint32_t frame = (uint32_t)(base / frame_pixels);
+    return { frame, (uint32_t)(base - (uint64_t)frame * frame_pixels) };
+}
+__device__ __forceinline__ const FrameDesc& locate(const PassArgs& a, Span span, uint32_t at, uint32_t frame_pixels,
+                                                   int& px, int& py)
+{
+    uint32_t offset = span.offset + at, frame = span.frame;
+    while (offset >= frame_pixels)
+    {
+        offset -= frame_pixels;
+        frame++;
+    }
+    const FrameDesc& f = a.frames[frame];
+    const uint32_t row = offset / (uint32_t)f.width;
+    py = (int)row;
+    px = (int)(offset - row * (uint32_t)f.width);
+    return f;
 }
 
 // The covered pixels of a warp's span, in order.
@@ -255,20 +266,20 @@ __device__ __forceinline__ int list_covered(const PassArgs& a, uint64_t base, in
     return n;
 }
 
-__global__ void __launch_bounds__(kThreads, 5) k_shade_visible(PassArgs a, uint64_t total, int rows, DiffMesh m,
-                                                            float4* out)
+__global__ void __launch_bounds__(kThreads, 5) k_shade_visible(PassArgs a, uint64_t total, uint32_t frame_pixels,
+                                                               int rows, DiffMesh m, float4* out)
 {
     __shared__ Covered s_list[kWarps];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t base = ((uint64_t)blockIdx.x * kWarps + warp) * (32u * (uint32_t)rows);
     const int n = list_covered(a, base, rows, total, m.nt, s_list[warp],
                                [&](uint64_t i) { out[i] = make_float4(0.f, 0.f, 0.f, 0.f); });
+    const Span span = span_of(base, frame_pixels);
     for (int b = (int)lane; b < n; b += 32)
     {
         const uint64_t i = base + s_list[warp].at[b];
-        const FrameDesc& f = a.frames[frame_of_pixel(a, i)];
-        const uint64_t local = i - f.pix_base;
-        const int px = (int)(local % (uint32_t)f.width), py = (int)(local / (uint32_t)f.width);
+        int px, py;
+        const FrameDesc& f = locate(a, span, s_list[warp].at[b], frame_pixels, px, py);
         PixelState s;
         float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
         if (pixel_forward(f, m, s_list[warp].tri[b], px, py, s))
@@ -317,14 +328,15 @@ __device__ __forceinline__ void add_packed(float* sums, uint32_t v, V3 da, V3 dn
 // 151, and k_shade_visible 118 -> 89.  4 blocks of 128 per SM (121 registers)
 // against 5 (96, 40 bytes spilled) measured 151 and 148 us, 6 157.
 template <bool Packed>
-__global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t total, int rows, DiffMesh m,
-                                                       const float4* grad, DiffGrads g)
+__global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t total, uint32_t frame_pixels, int rows,
+                                                          DiffMesh m, const float4* grad, DiffGrads g)
 {
     __shared__ Covered s_list[kWarps];
     __shared__ double red[kWarps][5];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t base = ((uint64_t)blockIdx.x * kWarps + warp) * (32u * (uint32_t)rows);
     const int n = list_covered(a, base, rows, total, m.nt, s_list[warp], [](uint64_t) {});
+    const Span span = span_of(base, frame_pixels);
     double sums[5] = { 0.0, 0.0, 0.0, 0.0, 0.0 };  // of the warp, lane 0
     for (int b0 = 0; b0 < n; b0 += 32)
     {
@@ -334,9 +346,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t t
         {
             const uint64_t i = base + s_list[warp].at[b0 + lane];
             const uint32_t tri = s_list[warp].tri[b0 + lane];
-            const FrameDesc& f = a.frames[frame_of_pixel(a, i)];
-            const uint64_t local = i - f.pix_base;
-            const int px = (int)(local % (uint32_t)f.width), py = (int)(local / (uint32_t)f.width);
+            int px, py;
+            const FrameDesc& f = locate(a, span, s_list[warp].at[b0 + lane], frame_pixels, px, py);
             PixelState s;
             if (pixel_forward(f, m, tri, px, py, s))
             {
@@ -369,13 +380,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t t
                     }
                     dNn = dNn + dnh * t.H;
                     const V3 dH = dnh * t.Nn;
-                    const V3 dHr = normalize_grad(t.H, t.hlen, dH);  // H = normalize(L + E)
+                    const V3 dHr = normalize_grad(t.H, t.hinv, dH);  // H = normalize(L + E)
                     dL = dL + dHr;
-                    const V3 dEr = normalize_grad(t.E, t.elen, dHr);  // E = normalize(eye - P)
+                    const V3 dEr = normalize_grad(t.E, t.einv, dHr);  // E = normalize(eye - P)
                     dP = dP - dEr;
                 }
-                const V3 dNraw = normalize_grad(t.Nn, t.nlen, dNn);
-                dl = normalize_grad(t.L, t.llen, dL);
+                const V3 dNraw = normalize_grad(t.Nn, t.ninv, dNn);
+                dl = normalize_grad(t.L, sh.light_inv, dL);
                 // P, N, A = sum b_k (p_k, n_k, a_k)
                 float db[3];
                 for (int k = 0; k < 3; k++)
@@ -491,8 +502,8 @@ cudaError_t launch_shade_visible(const PassArgs& a, uint64_t total, const DiffMe
 {
     const int rows = span_rows(a, total);
     if (total)
-        k_shade_visible<<<(unsigned)((total + kThreads * rows - 1) / (kThreads * rows)), kThreads, 0, s>>>(a, total, rows,
-                                                                                                          m, out);
+        k_shade_visible<<<(unsigned)((total + kThreads * rows - 1) / (kThreads * rows)), kThreads, 0, s>>>(
+            a, total, (uint32_t)(total / a.num_frames), rows, m, out);
     return cudaGetLastError();
 }
 
@@ -501,10 +512,11 @@ cudaError_t launch_backward(const PassArgs& a, uint64_t total, const DiffMesh& m
 {
     const int rows = span_rows(a, total);
     const unsigned blocks = (unsigned)((total + kThreads * rows - 1) / (kThreads * rows));
+    const uint32_t frame_pixels = (uint32_t)(total / a.num_frames);
     if (total && g.packed)
-        k_backward<true><<<blocks, kThreads, 0, s>>>(a, total, rows, m, grad, g);
+        k_backward<true><<<blocks, kThreads, 0, s>>>(a, total, frame_pixels, rows, m, grad, g);
     else if (total)
-        k_backward<false><<<blocks, kThreads, 0, s>>>(a, total, rows, m, grad, g);
+        k_backward<false><<<blocks, kThreads, 0, s>>>(a, total, frame_pixels, rows, m, grad, g);
     k_finish<<<g.packed ? (m.nv + kThreads - 1) / kThreads : 1, kThreads, 0, s>>>(g, m.nv);
     return cudaGetLastError();
 }

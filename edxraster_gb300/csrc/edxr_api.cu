@@ -144,6 +144,7 @@ void edxr::frame_shading(FrameDesc& f, int ps_kind, const float light[3], float 
         f.light[q] = (float)unit[q];
         f.light_lo[q] = (float)(unit[q] - (double)f.light[q]);
     }
+    f.light_inv = (float)(1.0 / ln);
     f.ks = ks;
     f.shininess = shininess;
 }
@@ -1186,8 +1187,12 @@ edxr_status diff_mesh(edxr_renderer* r, const edxr_mesh* mesh, const edxr_shader
     if (params)
     {
         m->override_shading = 1;
-        for (int q = 0; q < 3; q++)
-            m->light[q] = params->light[q];
+        const double lx = params->light[0], ly = params->light[1], lz = params->light[2];
+        const double ln = std::sqrt(lx * lx + ly * ly + lz * lz);
+        m->light[0] = (float)(lx / ln);
+        m->light[1] = (float)(ly / ln);
+        m->light[2] = (float)(lz / ln);
+        m->light_inv = (float)(1.0 / ln);
         m->ks = params->ks;
         m->shininess = params->shininess;
     }
