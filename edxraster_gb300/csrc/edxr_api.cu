@@ -1189,9 +1189,12 @@ edxr_status diff_mesh(edxr_renderer* r, const edxr_mesh* mesh, const edxr_shader
         m->override_shading = 1;
         const double lx = params->light[0], ly = params->light[1], lz = params->light[2];
         const double ln = std::sqrt(lx * lx + ly * ly + lz * lz);
-        m->light[0] = (float)(lx / ln);
-        m->light[1] = (float)(ly / ln);
-        m->light[2] = (float)(lz / ln);
+        const double unit[3] = { lx / ln, ly / ln, lz / ln };
+        for (int q = 0; q < 3; q++)
+        {
+            m->light[q] = (float)unit[q];
+            m->light_lo[q] = (float)(unit[q] - (double)m->light[q]);
+        }
         m->light_inv = (float)(1.0 / ln);
         m->ks = params->ks;
         m->shininess = params->shininess;

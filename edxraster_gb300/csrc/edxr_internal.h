@@ -243,7 +243,7 @@ struct DiffMesh
     uint32_t pos_stride, nrm_stride, alb_stride;
     uint32_t nv, nt;
     int override_shading;   // 1: use light/ks/shininess below for every frame
-    float light[3], light_inv, ks, shininess;  // light normalised, 1 / its length
+    float light[3], light_lo[3], light_inv, ks, shininess;  // unit light as float pairs, 1 / its length
 };
 constexpr int kPackedFloats = 12;  // per vertex: albedo, normal and position gradient, 3 unused
 struct DiffGrads
