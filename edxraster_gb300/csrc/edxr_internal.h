@@ -106,9 +106,9 @@ struct FrameDesc
 };
 
 // One triangle after clipping and setup (RasterTriangle, RasterTriangle.h:11-24),
-// 64 bytes, written by the setup kernel in any order; `order` restores the
+// 64 bytes (aligned so: read and written 32 at a time), written by the setup kernel in any order; `order` restores the
 // reference's submission order: input triangle * 16 + fan index.
-struct __align__(16) RTri
+struct __align__(64) RTri
 {
     int v0x, v0y, v1x, v1y;
     int v2x, v2y;

@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(256, 6) k_setup(PassArgs a)
         t.order = tri << 4;
         t.meta |= fi << 12;
         t.poly = kUnclipped;
-        a.rtris[gi] = t;
+        store_rtri(a.rtris + gi, t);
         a.rtri_zlo[gi] = zmin_key(t, wrap_free(t));
     }
     bin_big_append(a, gi, nOut && big);
@@ -504,7 +504,7 @@ __device__ __forceinline__ void clip_piece(const PassArgs& a, bool has, uint32_t
         tk.meta |= fi << 12;
         tk.poly = (poly << 4) | (fan + 1u);
         kept = true;
-        a.rtris[ri] = tk;
+        store_rtri(a.rtris + ri, tk);
         a.rtri_zlo[ri] = zmin_key(tk, wrap_free(tk));
         const BinGeom bg = bin_geom(tk, f);
         big = !bg.small;
@@ -1312,7 +1312,7 @@ __device__ __forceinline__ void stage_tri(const PassArgs& a, uint32_t entry, uin
         return;
     }
     const bool accept = (entry & 3u) == kDecisionAccept;
-    const RTri t = a.rtris[ri];
+    const RTri t = load_rtri(a.rtris + ri);
     const Edges e = tri_edges(t);
     // pixel (lx, ly) of the tile samples at (16*(16*tileX + lx) + 8, ...)
     const int ox = (tileX << 8) + 8, oy = (tileY << 8) + 8;
@@ -1518,7 +1518,7 @@ static __device__ __forceinline__ void write_pixel(const PixelOut a, const Frame
         a.tri_id[pix] = kNoTriangle;
         return;
     }
-    const RTri t = a.rtris[ri];
+    const RTri t = load_rtri(a.rtris + ri);
     const Edges e = tri_edges(t);
     const int cx = (px << 4) + 8, cy = (py << 4) + 8;
     const int n1 = wadd(wmul(e.B[1], wsub(cx, t.v2x)), wmul(e.C[1], wsub(cy, t.v2y)));
@@ -1549,7 +1549,7 @@ static __device__ __forceinline__ void write_pixel_fast(const PixelOut a, const 
     const uint32_t tri = ((rank - 1u) >> 4) - f.tri_base;
     const uint32_t* idx = f.indices + 3 * (size_t)tri;
     const uint32_t vi[3] = { __ldg(idx), __ldg(idx + 1), __ldg(idx + 2) };
-    const RTri t = a.rtris[ri];
+    const RTri t = load_rtri(a.rtris + ri);
     float L0, L1;
     const float d = depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
     const float3 c = shade_common<true>(f, t, a.polys, L0, L1, vi);
@@ -2141,7 +2141,7 @@ static __device__ __forceinline__ void write_pixel_ms(const PassArgs& a, const F
         uint32_t id = kNoTriangle, rgb = 0;
         if (ri != kNoTriangle)
         {
-            const RTri t = a.rtris[ri];
+            const RTri t = load_rtri(a.rtris + ri);
             id = t.order >> 4;
             float L0, L1;
             depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
