@@ -261,7 +261,13 @@ __device__ __forceinline__ uint32_t frame_of_triangle(const PassArgs& a, uint32_
 // A small set-up triangle is binned here as well.  A set-up triangle's
 // record goes to its own slot (no append); the clip queue and the warp's
 // stripe of the unsorted bin list take one atomic per warp each.
-__global__ void __launch_bounds__(256, 6) k_setup(PassArgs a)
+// Blocks of 128: warps of culled triangles leave early, and a small block's
+// place is refilled sooner.  256 batched views 147 -> 142 us at 256 threads,
+// 6 blocks per SM, against 128, 12 (64, 24: 149; 48 registers without the 24
+// spilled bytes: 160 and 153).
+constexpr int kSetupThreads = 128;
+
+__global__ void __launch_bounds__(kSetupThreads, 12) k_setup(PassArgs a)
 {
     follow_on();
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2751,7 +2757,7 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
     mark(1);
     if (a.total_tris)
     {
-        go(k_setup, (a.total_tris + 255) / 256, 256, 0);
+        go(k_setup, (a.total_tris + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0);
         // (no more blocks than one 16-lane group per triangle fills)
         go(k_clip, min((uint32_t)sms * 8u, (a.total_tris + 7u) / 8u), kClipThreads, 0);
     }
