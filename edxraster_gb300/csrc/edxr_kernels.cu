@@ -796,6 +796,7 @@ __global__ void __launch_bounds__(256) k_bin_move(PassArgs a)
     {
         const uint32_t j = rd * stride + blockIdx.x * blockDim.x + threadIdx.x;
         uint2 e = make_uint2(kEmptySlot, 0u);
+        uint32_t bin = 0;  // the bin's start, loaded beside the occluder bound
         if (j < total)
         {
             // stripe of entry j: the last one starting at or before it
@@ -810,6 +811,7 @@ __global__ void __launch_bounds__(256) k_bin_move(PassArgs a)
             if (e.x != kEmptySlot)
             {
                 const uint32_t zocc = a.tile_zocc[e.x];
+                bin = a.tile_offset[e.x];
                 const uint32_t ri = e.y >> 2;
                 if (zocc != 0xFFFFFFFFu && ri < a.rtri_capacity && a.rtri_zlo[ri] > min(zocc, 0xBF800000u))
                     e.x = kEmptySlot;
@@ -845,7 +847,7 @@ __global__ void __launch_bounds__(256) k_bin_move(PassArgs a)
         }
         if (e.x == kEmptySlot)
             continue;
-        const uint64_t pos = (uint64_t)a.tile_offset[e.x] + base;
+        const uint64_t pos = (uint64_t)bin + base;
         if (pos < a.bin_capacity)
             a.bins[pos] = e.y;
     }
