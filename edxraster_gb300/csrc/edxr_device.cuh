@@ -1053,4 +1053,23 @@ __device__ __forceinline__ uint32_t find_frame(const FrameDesc* frames, uint32_t
     return lo;
 }
 
+// find_frame of one index by a whole warp: 32 frames are compared at a time,
+// so 1024 frames take two rounds of one load instead of ten dependent loads.
+template <typename Get>
+__device__ __forceinline__ uint32_t find_frame_warp(const FrameDesc* frames, uint32_t n, uint32_t i, Get get)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, len = n;
+    while (len > 1)
+    {
+        const uint32_t step = (len + 31) / 32;
+        const bool at = lane * step < len && get(frames[lo + lane * step]) <= i;
+        const uint32_t m = __ballot_sync(0xffffffffu, at);
+        const uint32_t k = m ? 31u - (uint32_t)__clz(m) : 0u;
+        lo += k * step;
+        len = min(step, len - k * step);
+    }
+    return lo;
+}
+
 }  // namespace edxr

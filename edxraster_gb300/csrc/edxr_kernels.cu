@@ -69,9 +69,17 @@ __global__ void k_clear(PassArgs a)
     follow_on();
     const uint32_t stride = gridDim.x * blockDim.x;
     if (a.vrecs)
-        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.total_vertices; i += stride)
+        for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < a.total_vertices; i0 += stride)
         {
-            const uint32_t fi = find_frame(a.frames, a.num_frames, i, [](const FrameDesc& f) { return f.vtx_base; });
+            // the frame of the warp's first vertex, then on over the frames
+            // that start at or before the lane's own
+            const auto base = [](const FrameDesc& f) { return f.vtx_base; };
+            uint32_t fi = find_frame_warp(a.frames, a.num_frames, i0, base);
+            const uint32_t i = i0 + (threadIdx.x & 31);
+            if (i >= a.total_vertices)
+                break;
+            while (fi + 1 < a.num_frames && a.frames[fi + 1].vtx_base <= i)
+                fi++;
             const FrameDesc& f = a.frames[fi];
             a.vrecs[i] = vertex_record(f, i - f.vtx_base);
         }
