@@ -2153,15 +2153,23 @@ static __device__ __forceinline__ void write_pixel_ms(const PassArgs& a, const F
     {
         // the next sample's winner, shaded once for every sample it wins
         const uint32_t low = low_words[512 * (__ffs(todo) - 1)];
-        const uint32_t ri = raster_triangle_of(a, less ? low : ~low, nr);
+        const uint32_t rank = less ? low : ~low;
+        const uint32_t ri = raster_triangle_of(a, rank, nr);
         uint32_t id = kNoTriangle, rgb = 0;
         if (ri != kNoTriangle)
         {
+            // the rank names the input triangle: its indices load beside its record
+            id = ((rank - 1u) >> 4) - f.tri_base;
+            uint32_t vi[3];
+            if (Common)
+            {
+                const uint32_t* idx = f.indices + 3 * (size_t)id;
+                vi[0] = __ldg(idx); vi[1] = __ldg(idx + 1); vi[2] = __ldg(idx + 2);
+            }
             const RTri t = load_rtri(a.rtris + ri);
-            id = t.order >> 4;
             float L0, L1;
             depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
-            const float3 c = Common ? shade_common<true>(f, t, a.polys, L0, L1)
+            const float3 c = Common ? shade_common<true>(f, t, a.polys, L0, L1, vi)
                                     : shade_slow(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
             rgb = to_byte(c.x) | (to_byte(c.y) << 8) | (to_byte(c.z) << 16);
         }
