@@ -15,9 +15,10 @@
 //   one the raster kernel uses, edxr_device.cuh shade_model).
 // Adjoint (k_backward): the same recomputation, then reverse-mode through
 // the shading model, the interpolation, the barycentric solve and the MVP
-// transform.  Per-vertex gradients are accumulated with float atomics; the
-// light, ks and shininess gradients are reduced per block and accumulated in
-// double.  Nothing per pixel is stored between the passes.
+// transform.  Per-vertex gradients are accumulated with float reductions (in
+// packed scratch sums that k_finish adds to the caller's arrays, or straight
+// there); the light, ks and shininess gradients in float pairs per lane and in
+// double over the blocks.  Nothing per pixel is stored between the passes.
 #include <cuda_runtime.h>
 
 #include "edxr_device.cuh"
@@ -42,18 +43,8 @@ __device__ __forceinline__ V3 v3(float x, float y, float z) { return { x, y, z }
 __device__ __forceinline__ V3 operator+(V3 a, V3 b) { return { a.x + b.x, a.y + b.y, a.z + b.z }; }
 __device__ __forceinline__ V3 operator-(V3 a, V3 b) { return { a.x - b.x, a.y - b.y, a.z - b.z }; }
 __device__ __forceinline__ V3 operator*(float s, V3 a) { return { s * a.x, s * a.y, s * a.z }; }
-// Products are added with one rounding (the library is built without
-// contraction, so a fused multiply-add is written out).
-__device__ __forceinline__ float dot(V3 a, V3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
-__device__ __forceinline__ V3 fma3(float s, V3 a, V3 c) { return { fmaf(s, a.x, c.x), fmaf(s, a.y, c.y), fmaf(s, a.z, c.z) }; }
-// 1 / |a|: the hardware estimate and one Newton step on its residual; an
-// estimate that is not finite (a zero or overflowing square) stays as it is.
-__device__ __forceinline__ float inv_len(V3 a)
-{
-    const float x = dot(a, a), y = rsqrtf(x);
-    const float e = x > 0.0f && x < 3.0e38f ? fmaf(-(x * y), y, 1.0f) : 0.0f;
-    return fmaf(0.5f * y, e, y);
-}
+__device__ __forceinline__ float dot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ float inv_len(V3 a) { return 1.0f / sqrtf(dot(a, a)); }
 __device__ __forceinline__ V3 ld(const char* base, uint32_t stride, uint32_t i, float dflt)
 {
     if (!base)
@@ -62,20 +53,34 @@ __device__ __forceinline__ V3 ld(const char* base, uint32_t stride, uint32_t i, 
     return v3(__ldg(p), __ldg(p + 1), __ldg(p + 2));
 }
 // gradient of y = normalize(x) applied to dy: (dy - y (y . dy)) / |x|
-__device__ __forceinline__ V3 normalize_grad(V3 y, float invx, V3 dy) { return invx * fma3(-dot(y, dy), y, dy); }
+__device__ __forceinline__ V3 normalize_grad(V3 y, float invx, V3 dy) { return invx * (dy - dot(y, dy) * y); }
 
-// m0 x + m1 y + m2 z + m3 as a pair.
-__device__ __forceinline__ FF ff_dot4(float m0, float m1, float m2, float m3, float x, float y, float z)
+// Pairs of the barycentric solve, renormalised after every operation and with
+// no product fused beyond the exact remainders: where a triangle is seen
+// edge-on the solve cancels nearly all 48 bits, and the order of the roundings
+// is then part of the result.
+__device__ __forceinline__ FF pair_add(FF x, FF y) { return ff_norm(ff_sum(x, y)); }
+__device__ __forceinline__ FF pair_sub(FF x, FF y) { return pair_add(x, ff_neg(y)); }
+__device__ __forceinline__ FF pair_mul(FF x, FF y)
 {
-    const FF p = two_prod(m0, x), q = two_prod(m1, y), r = two_prod(m2, z);
-    const FF s = two_sum(p.hi, q.hi), t = two_sum(r.hi, m3), u = two_sum(s.hi, t.hi);
-    return quick_two_sum(u.hi, u.lo + ((s.lo + t.lo) + ((p.lo + q.lo) + r.lo)));
+    const FF p = two_prod(x.hi, y.hi);
+    return quick_two_sum(p.hi, p.lo + (x.hi * y.lo + x.lo * y.hi));
+}
+__device__ __forceinline__ FF pair_mul_f(FF x, float y)
+{
+    const FF p = two_prod(x.hi, y);
+    return quick_two_sum(p.hi, p.lo + x.lo * y);
+}
+// m0 x + m1 y + m2 z + m3 as a pair.
+__device__ __forceinline__ FF pair_dot4(float m0, float m1, float m2, float m3, float x, float y, float z)
+{
+    return pair_add(pair_add(two_prod(m0, x), two_prod(m1, y)), pair_add(two_prod(m2, z), { m3, 0.0f }));
 }
 // Everything the forward computes for one pixel, kept for the adjoint.
 struct PixelState
 {
     uint32_t vi[3];
-    V3 p[3], n[3], a[3];  // [0]: of vertex 0; [k]: of vertex k less that
+    V3 p[3], n[3], a[3];
     float ac[3], cc[3];
     float bt[3], S, b[3];
     float u, v;
@@ -97,68 +102,44 @@ __device__ __forceinline__ bool pixel_forward(const FrameDesc& f, const DiffMesh
         s.a[k] = ld(m.albedo, m.alb_stride, s.vi[k], 1.0f);
     }
     // The solve cancels heavily: a_k, c_k are the small projected distances of
-    // the vertices from the pixel centre, each a difference of O(1) terms, and
-    // thin triangles' cross products cancel again.  It is therefore carried in
+    // the vertices from the pixel centre, each a difference of O(1) terms.
+    // The clip coordinates and the pixel centre are therefore carried as
     // float pairs (hi + lo, about 48 bits; error-free products and sums,
-    // Dekker 1971 / Knuth), each result rounded to float once, without the
-    // FP64 unit (slow on this GPU).  Only vertex 0 is projected; the other two
-    // enter by their edges, exact differences of the positions and much
-    // shorter than them, along the pixel's rows (M0 - u M3, M1 - v M3): the
-    // pairs' error is then that of the edges and not of the positions (a
-    // thirtieth on a torus of 50,000 triangles).
+    // Dekker 1971 / Knuth), and so are a_k, c_k, the cross products and their
+    // sum, each rounded to float once: FP32 arithmetic throughout, accurate
+    // to a few float ulps of the results, without the FP64 unit (slow on
+    // this GPU).
     const float* M = f.mvp;
+    FF X[3], Y[3], Wd[3];
+    for (int k = 0; k < 3; k++)
+    {
+        const float x = s.p[k].x, y = s.p[k].y, z = s.p[k].z;
+        X[k] = pair_dot4(M[0], M[1], M[2], M[3], x, y, z);
+        Y[k] = pair_dot4(M[4], M[5], M[6], M[7], x, y, z);
+        Wd[k] = pair_dot4(M[12], M[13], M[14], M[15], x, y, z);
+    }
     const float rx = (float)px + 0.5f, ry = (float)py + 0.5f;  // exact
     const float* Rh = f.ndc_from_raster;
     const float* Rl = f.ndc_from_raster_lo;
-    const FF u = ff_norm(ff_sum(ff_sum(ff_prod_f({ Rh[0], Rl[0] }, rx), ff_prod_f({ Rh[1], Rl[1] }, ry)),
-                                { Rh[2], Rl[2] }));
-    const FF v = ff_norm(ff_sum(ff_sum(ff_prod_f({ Rh[3], Rl[3] }, rx), ff_prod_f({ Rh[4], Rl[4] }, ry)),
-                                { Rh[5], Rl[5] }));
+    const FF u = pair_add(pair_add(pair_mul_f({ Rh[0], Rl[0] }, rx), pair_mul_f({ Rh[1], Rl[1] }, ry)), { Rh[2], Rl[2] });
+    const FF v = pair_add(pair_add(pair_mul_f({ Rh[3], Rl[3] }, rx), pair_mul_f({ Rh[4], Rl[4] }, ry)), { Rh[5], Rl[5] });
     s.u = u.hi + u.lo;
     s.v = v.hi + v.lo;
-    FF a0, c0;
+    FF ac[3], cc[3];
+    for (int k = 0; k < 3; k++)
     {
-        const float x = s.p[0].x, y = s.p[0].y, z = s.p[0].z;
-        const FF X = ff_dot4(M[0], M[1], M[2], M[3], x, y, z);
-        const FF Y = ff_dot4(M[4], M[5], M[6], M[7], x, y, z);
-        const FF W = ff_dot4(M[12], M[13], M[14], M[15], x, y, z);
-        a0 = ff_norm(ff_sum(X, ff_neg(ff_prod(u, W))));
-        c0 = ff_norm(ff_sum(Y, ff_neg(ff_prod(v, W))));
+        ac[k] = pair_sub(X[k], pair_mul(u, Wd[k]));
+        cc[k] = pair_sub(Y[k], pair_mul(v, Wd[k]));
+        s.ac[k] = ac[k].hi + ac[k].lo;
+        s.cc[k] = cc[k].hi + cc[k].lo;
     }
-    FF ra[3], rc[3], da[2], dc[2];  // the rows; a_k - a_0 and c_k - c_0 for k = 1, 2
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-    {
-        ra[j] = ff_norm(ff_sum({ M[j], 0.0f }, ff_neg(ff_prod_f(u, M[12 + j]))));
-        rc[j] = ff_norm(ff_sum({ M[4 + j], 0.0f }, ff_neg(ff_prod_f(v, M[12 + j]))));
-    }
-#pragma unroll
-    for (int k = 0; k < 2; k++)
-    {
-        const V3 p = s.p[k + 1];
-        const FF e[3] = { two_sum(p.x, -s.p[0].x), two_sum(p.y, -s.p[0].y), two_sum(p.z, -s.p[0].z) };
-        da[k] = ff_dot3(ra, e);
-        dc[k] = ff_dot3(rc, e);
-        s.p[k + 1] = v3(e[0].hi, e[1].hi, e[2].hi);
-        s.n[k + 1] = s.n[k + 1] - s.n[0];
-        s.a[k + 1] = s.a[k + 1] - s.a[0];
-    }
-    s.ac[0] = a0.hi;
-    s.cc[0] = c0.hi;
-#pragma unroll
-    for (int k = 0; k < 2; k++)
-    {
-        const FF a1 = ff_sum(a0, da[k]), c1 = ff_sum(c0, dc[k]);
-        s.ac[k + 1] = a1.hi + a1.lo;
-        s.cc[k + 1] = c1.hi + c1.lo;
-    }
-    // the cross products a x c and their sum, with the products of a_0 and c_0
-    // that cancel left out: S = da_1 dc_2 - da_2 dc_1
-    const FF Sf = ff_norm(ff_sum(ff_prod(da[0], dc[1]), ff_neg(ff_prod(da[1], dc[0]))));
+    // the cross products and their sum stay pairs too: near an edge, or on a
+    // thin triangle, they cancel again
     FF bt[3];
-    bt[1] = ff_norm(ff_sum(ff_prod(da[1], c0), ff_neg(ff_prod(a0, dc[1]))));
-    bt[2] = ff_norm(ff_sum(ff_prod(a0, dc[0]), ff_neg(ff_prod(da[0], c0))));
-    bt[0] = ff_norm(ff_sum(ff_sum(Sf, ff_neg(bt[1])), ff_neg(bt[2])));
+    bt[0] = pair_sub(pair_mul(ac[1], cc[2]), pair_mul(ac[2], cc[1]));
+    bt[1] = pair_sub(pair_mul(ac[2], cc[0]), pair_mul(ac[0], cc[2]));
+    bt[2] = pair_sub(pair_mul(ac[0], cc[1]), pair_mul(ac[1], cc[0]));
+    const FF Sf = pair_add(pair_add(bt[0], bt[1]), bt[2]);
     const float S = Sf.hi + Sf.lo;
     if (!(S != 0.0f) || !(fabsf(S) < 3.0e38f))
         return false;
@@ -168,11 +149,9 @@ __device__ __forceinline__ bool pixel_forward(const FrameDesc& f, const DiffMesh
         s.bt[k] = bt[k].hi + bt[k].lo;
         s.b[k] = s.bt[k] / S;
     }
-    // (from vertex 0 along the edges: a pixel centre far outside a thin
-    // triangle has large weights, whose roundings then enter by the edges)
-    s.P = fma3(s.b[1], s.p[1], fma3(s.b[2], s.p[2], s.p[0]));
-    s.Nraw = fma3(s.b[1], s.n[1], fma3(s.b[2], s.n[2], s.n[0]));
-    s.A = fma3(s.b[1], s.a[1], fma3(s.b[2], s.a[2], s.a[0]));
+    s.P = s.b[0] * s.p[0] + s.b[1] * s.p[1] + s.b[2] * s.p[2];
+    s.Nraw = s.b[0] * s.n[0] + s.b[1] * s.n[1] + s.b[2] * s.n[2];
+    s.A = s.b[0] * s.a[0] + s.b[1] * s.a[1] + s.b[2] * s.a[2];
     return true;
 }
 
@@ -188,15 +167,13 @@ struct ShadeTerms
 // Light (normalised, and 1 / its length), ks and shininess in effect for frame f.
 struct Shading
 {
-    float light[3], light_lo[3], light_inv, ks, shininess;
+    float light[3], light_inv, ks, shininess;
 };
 __device__ __forceinline__ Shading shading_of(const FrameDesc& f, const DiffMesh& m)
 {
     if (m.override_shading)
-        return { { m.light[0], m.light[1], m.light[2] }, { m.light_lo[0], m.light_lo[1], m.light_lo[2] }, m.light_inv,
-                 m.ks, m.shininess };
-    return { { f.light[0], f.light[1], f.light[2] }, { f.light_lo[0], f.light_lo[1], f.light_lo[2] }, f.light_inv, f.ks,
-             f.shininess };
+        return { { m.light[0], m.light[1], m.light[2] }, m.light_inv, m.ks, m.shininess };
+    return { { f.light_unit[0], f.light_unit[1], f.light_unit[2] }, f.light_inv, f.ks, f.shininess };
 }
 
 __device__ __forceinline__ V3 shade_forward(const FrameDesc& f, const Shading& sh, const PixelState& s,
@@ -213,21 +190,19 @@ __device__ __forceinline__ V3 shade_forward(const FrameDesc& f, const Shading& s
     t.spec = 0.0f;
     if (t.specular)
     {
-        const V3 Er = (v3(f.eye[0], f.eye[1], f.eye[2]) - s.P) + v3(f.eye_lo[0], f.eye_lo[1], f.eye_lo[2]);
+        const V3 Er = v3(f.eye[0], f.eye[1], f.eye[2]) - s.P;
         t.einv = inv_len(Er);
         t.E = t.einv * Er;
-        const V3 Hr = fma3(t.einv, Er, t.L);
+        const V3 Hr = t.L + t.E;
         t.hinv = inv_len(Hr);
         t.H = t.hinv * Hr;
-        // (of the vectors before normalisation: the exponent amplifies every
-        // rounding of N.H)
-        t.nh = dot(s.Nraw, Hr) * (t.ninv * t.hinv);
+        t.nh = dot(t.Nn, t.H);
         t.nhc = t.clamp ? fmaxf(t.nh, 0.0f) : t.nh;
         t.powv = powf(t.nhc, sh.shininess);
         t.spec = sh.ks * t.powv;
     }
     if (t.albedo)
-        return fma3(t.diffuse, s.A, v3(t.spec, t.spec, t.spec));
+        return v3(s.A.x * t.diffuse + t.spec, s.A.y * t.diffuse + t.spec, s.A.z * t.diffuse + t.spec);
     return v3(t.diffuse + t.spec, t.diffuse + t.spec, t.diffuse + t.spec);
 }
 
@@ -355,9 +330,10 @@ __device__ __forceinline__ void add_packed(float* sums, uint32_t v, V3 da, V3 dn
 // reductions a vertex.  The reductions bounded the kernel: 50,000 triangles
 // in 64 views of 256x256, 1.3 M covered pixels, 51 M reduction sectors in L2,
 // 311 us; packed 236; with the covered pixels of a span listed first (and
-// one double reduction of the global sums per 1,024 pixels instead of 256)
-// 151, and k_shade_visible 118 -> 89.  4 blocks of 128 per SM (121 registers)
-// against 5 (96, 40 bytes spilled) measured 151 and 148 us, 6 157.
+// one double reduction of the global sums per block) and no 64-bit division
+// per pixel 138, and k_shade_visible 118 -> 88.  What is left is the solve's
+// arithmetic.  4 blocks of 128 per SM against 5 (some spilled) measured 151 and
+// 148 us before the divisions went, 6 157.
 template <bool Packed>
 __global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t total, uint32_t frame_pixels, int rows,
                                                           DiffMesh m, const float4* grad, DiffGrads g)
@@ -368,7 +344,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t t
     const uint64_t base = ((uint64_t)blockIdx.x * kWarps + warp) * (32u * (uint32_t)rows);
     const int n = list_covered(a, base, rows, total, m.nt, s_list[warp], [](uint64_t) {});
     const Span span = span_of(base, frame_pixels);
-    double sums[5] = { 0.0, 0.0, 0.0, 0.0, 0.0 };  // of the warp, lane 0
+    // The five global gradients are sums of large terms of both signs: each lane
+    // keeps them as pairs, so that the order of the pixels leaves no trace.
+    FF sums[5] = {};
     for (int b0 = 0; b0 < n; b0 += 32)
     {
         V3 dl = v3(0.f, 0.f, 0.f);
@@ -394,8 +372,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t t
                 V3 dNn = v3(0.f, 0.f, 0.f), dL = v3(0.f, 0.f, 0.f), dP = v3(0.f, 0.f, 0.f);
                 // diffuse = (max(nl, 0) + 0.2) * 3/pi
                 const float dnl = (t.nl > 0.0f) ? ddiff * 0.954929658551372f : 0.0f;
-                dL = fma3(dnl, t.Nn, dL);
-                dNn = fma3(dnl, t.L, dNn);
+                dL = dL + dnl * t.Nn;
+                dNn = dNn + dnl * t.L;
                 if (t.specular)
                 {
                     // spec = ks * nhc^s
@@ -404,12 +382,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t t
                         dshin = dspec * sh.ks * t.powv * logf(t.nhc);
                     float dnh = 0.0f;
                     if (!t.clamp || t.nh > 0.0f)
-                    {
-                        // nhc^(s - 1) from nhc^s where that is far from underflow
-                        const float p1 = fabsf(t.powv) > 1e-30f ? t.powv / t.nhc : powf(t.nhc, sh.shininess - 1.0f);
-                        dnh = (sh.shininess == 0.0f) ? 0.0f : dspec * sh.ks * sh.shininess * p1;
-                    }
-                    dNn = fma3(dnh, t.H, dNn);
+                        dnh = (sh.shininess == 0.0f)
+                                  ? 0.0f
+                                  : dspec * sh.ks * sh.shininess * powf(t.nhc, sh.shininess - 1.0f);
+                    dNn = dNn + dnh * t.H;
                     const V3 dH = dnh * t.Nn;
                     const V3 dHr = normalize_grad(t.H, t.hinv, dH);  // H = normalize(L + E)
                     dL = dL + dHr;
@@ -417,37 +393,32 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t t
                     dP = dP - dEr;
                 }
                 const V3 dNraw = normalize_grad(t.Nn, t.ninv, dNn);
-                // with the unit light as a pair: its rounding to float would
-                // leave the same share of (L . dL) L in every pixel's term
-                const V3 lo = v3(sh.light_lo[0], sh.light_lo[1], sh.light_lo[2]);
-                const float along = dot(t.L, dL) + dot(lo, dL);
-                dl = sh.light_inv * fma3(-along, lo, fma3(-along, t.L, dL));
+                dl = normalize_grad(t.L, sh.light_inv, dL);
                 // P, N, A = sum b_k (p_k, n_k, a_k)
-                // by vertices 1 and 2 relative to vertex 0 (its weight is 1 less theirs)
-                float db[3] = { 0.0f, 0.0f, 0.0f };
-                for (int k = 1; k < 3; k++)
+                float db[3];
+                for (int k = 0; k < 3; k++)
                     db[k] = dot(dP, s.p[k]) + dot(dNraw, s.n[k]) + dot(dA, s.a[k]);
                 // b = bt / S
-                const float bdb = fmaf(s.b[1], db[1], s.b[2] * db[2]);
+                const float bdb = s.b[0] * db[0] + s.b[1] * db[1] + s.b[2] * db[2];
                 float dbt[3];
                 for (int k = 0; k < 3; k++)
                     dbt[k] = (db[k] - bdb) / s.S;
                 // bt = a x c
-                const float dac[3] = { fmaf(dbt[2], s.cc[1], -(dbt[1] * s.cc[2])), fmaf(dbt[0], s.cc[2], -(dbt[2] * s.cc[0])),
-                                       fmaf(dbt[1], s.cc[0], -(dbt[0] * s.cc[1])) };
-                const float dcc[3] = { fmaf(dbt[1], s.ac[2], -(dbt[2] * s.ac[1])), fmaf(dbt[2], s.ac[0], -(dbt[0] * s.ac[2])),
-                                       fmaf(dbt[0], s.ac[1], -(dbt[1] * s.ac[0])) };
+                float dac[3] = { 0.f, 0.f, 0.f }, dcc[3] = { 0.f, 0.f, 0.f };
+                dac[1] += dbt[0] * s.cc[2]; dcc[2] += dbt[0] * s.ac[1]; dac[2] -= dbt[0] * s.cc[1]; dcc[1] -= dbt[0] * s.ac[2];
+                dac[2] += dbt[1] * s.cc[0]; dcc[0] += dbt[1] * s.ac[2]; dac[0] -= dbt[1] * s.cc[2]; dcc[2] -= dbt[1] * s.ac[0];
+                dac[0] += dbt[2] * s.cc[1]; dcc[1] += dbt[2] * s.ac[0]; dac[1] -= dbt[2] * s.cc[0]; dcc[0] -= dbt[2] * s.ac[1];
                 // a_k = X_k - u W_k, c_k = Y_k - v W_k, (X, Y, W) = rows 0, 1, 3 of MVP (p, 1)
                 for (int k = 0; k < 3; k++)
                 {
                     V3 dp = v3(0.f, 0.f, 0.f);
                     if (g.positions)
                     {
-                        const float dX = dac[k], dY = dcc[k], dW = fmaf(-s.u, dac[k], -(s.v * dcc[k]));
+                        const float dX = dac[k], dY = dcc[k], dW = -s.u * dac[k] - s.v * dcc[k];
                         const float* M = f.mvp;
-                        dp = v3(fmaf(M[0], dX, fmaf(M[4], dY, M[12] * dW)), fmaf(M[1], dX, fmaf(M[5], dY, M[13] * dW)),
-                                fmaf(M[2], dX, fmaf(M[6], dY, M[14] * dW)));
-                        dp = fma3(s.b[k], dP, dp);
+                        dp = v3(M[0] * dX + M[4] * dY + M[12] * dW, M[1] * dX + M[5] * dY + M[13] * dW,
+                                M[2] * dX + M[6] * dY + M[14] * dW);
+                        dp = dp + s.b[k] * dP;
                     }
                     if (Packed)
                         add_packed(g.packed, s.vi[k], s.b[k] * dA, s.b[k] * dNraw, dp);
@@ -460,21 +431,25 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward(PassArgs a, uint64_t t
                 }
             }
         }
-        // the five global gradients: summed over the warp, then in double
-        float vals[5] = { dl.x, dl.y, dl.z, dks, dshin };
+        const float vals[5] = { dl.x, dl.y, dl.z, dks, dshin };
 #pragma unroll
         for (int q = 0; q < 5; q++)
         {
-            for (int o = 16; o > 0; o >>= 1)
-                vals[q] += __shfl_down_sync(0xffffffffu, vals[q], o);
-            if (lane == 0)
-                sums[q] += (double)vals[q];
+            const FF t = two_sum(sums[q].hi, vals[q]);
+            sums[q] = { t.hi, sums[q].lo + t.lo };
         }
     }
+    if (n > 0)
+#pragma unroll
+        for (int q = 0; q < 5; q++)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                sums[q] = ff_sum(sums[q], { __shfl_down_sync(0xffffffffu, sums[q].hi, o),
+                                            __shfl_down_sync(0xffffffffu, sums[q].lo, o) });
     if (lane == 0)
 #pragma unroll
         for (int q = 0; q < 5; q++)
-            red[warp][q] = sums[q];
+            red[warp][q] = fabsf(sums[q].hi) < INFINITY ? (double)sums[q].hi + (double)sums[q].lo : (double)sums[q].hi;
     __syncthreads();
     if (threadIdx.x < 5)
     {

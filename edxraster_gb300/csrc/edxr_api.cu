@@ -79,6 +79,18 @@ bool edxr::eye_from_mv(const float* mv, double eye[3])
     return true;
 }
 
+// v normalised in float, (1 / |v|) v with every operation rounded (kept in a
+// volatile: a host compiler may contract products and sums otherwise).
+static void normalize_float(const float v[3], float unit[3], float& inv)
+{
+    auto mul = [](float a, float b) { volatile float r = a * b; return r; };
+    const float x = mul(v[0], v[0]), y = mul(v[1], v[1]), z = mul(v[2], v[2]);
+    const float len = std::sqrt((x + y) + z);
+    inv = 1.0f / len;
+    for (int q = 0; q < 3; q++)
+        unit[q] = mul(inv, v[q]);
+}
+
 void edxr::frame_camera(FrameDesc& f, const float mv[16], const float proj[16], const float raster[16])
 {
     mat_mul(proj, mv, f.mvp);
@@ -144,7 +156,7 @@ void edxr::frame_shading(FrameDesc& f, int ps_kind, const float light[3], float 
         f.light[q] = (float)unit[q];
         f.light_lo[q] = (float)(unit[q] - (double)f.light[q]);
     }
-    f.light_inv = (float)(1.0 / ln);
+    normalize_float(f.light_raw, f.light_unit, f.light_inv);
     f.ks = ks;
     f.shininess = shininess;
 }
@@ -1187,15 +1199,7 @@ edxr_status diff_mesh(edxr_renderer* r, const edxr_mesh* mesh, const edxr_shader
     if (params)
     {
         m->override_shading = 1;
-        const double lx = params->light[0], ly = params->light[1], lz = params->light[2];
-        const double ln = std::sqrt(lx * lx + ly * ly + lz * lz);
-        const double unit[3] = { lx / ln, ly / ln, lz / ln };
-        for (int q = 0; q < 3; q++)
-        {
-            m->light[q] = (float)unit[q];
-            m->light_lo[q] = (float)(unit[q] - (double)m->light[q]);
-        }
-        m->light_inv = (float)(1.0 / ln);
+        normalize_float(params->light, m->light, m->light_inv);
         m->ks = params->ks;
         m->shininess = params->shininess;
     }

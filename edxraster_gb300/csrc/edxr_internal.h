@@ -95,8 +95,7 @@ struct FrameDesc
     double ndc_from_raster_d[6];  // the raster-to-NDC inverse in double (differentiable form)
     float ndc_from_raster_lo[6];  // ndc_from_raster_d - ndc_from_raster: with it, a float pair (hi + lo)
     float eye_lo[3], light_lo[3]; // eye_d - eye and the normalised light's remainder: float pairs with eye and light
-    float light_inv;              // 1 / the length of the light direction as given
-    float pad3;
+    float light_unit[3], light_inv; // light_raw normalised in float and 1 / its length (differentiable form)
     // textures of the textured Lambertian shader
     const uint32_t* tex_ids;      // per input triangle (NULL: slot 0)
     const TexDesc* textures;
@@ -243,7 +242,7 @@ struct DiffMesh
     uint32_t pos_stride, nrm_stride, alb_stride;
     uint32_t nv, nt;
     int override_shading;   // 1: use light/ks/shininess below for every frame
-    float light[3], light_lo[3], light_inv, ks, shininess;  // unit light as float pairs, 1 / its length
+    float light[3], light_inv, ks, shininess;  // light normalised, 1 / its length
 };
 constexpr int kPackedFloats = 12;  // per vertex: albedo, normal and position gradient, 3 unused
 struct DiffGrads
