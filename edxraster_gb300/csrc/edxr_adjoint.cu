@@ -272,7 +272,10 @@ __device__ __forceinline__ int list_covered(const PassArgs& a, uint64_t base, in
     return n;
 }
 
-__global__ void __launch_bounds__(kThreads, 5) k_shade_visible(PassArgs a, uint64_t total, uint32_t frame_pixels,
+// Bound by the chain indices -> vertices -> solve and the solve's arithmetic:
+// 6 blocks of 128 per SM (80 registers) 84.4 us on 50,000 triangles in 64 views
+// of 256x256, 5 (91) 87, 8 (64, spilled) 90.
+__global__ void __launch_bounds__(kThreads, 6) k_shade_visible(PassArgs a, uint64_t total, uint32_t frame_pixels,
                                                                int rows, DiffMesh m, float4* out)
 {
     __shared__ Covered s_list[kWarps];
@@ -331,7 +334,7 @@ __device__ __forceinline__ void add_packed(float* sums, uint32_t v, V3 da, V3 dn
 // in 64 views of 256x256, 1.3 M covered pixels, 51 M reduction sectors in L2,
 // 311 us; packed 236; with the covered pixels of a span listed first (and
 // one double reduction of the global sums per block) and no 64-bit division
-// per pixel 138, and k_shade_visible 118 -> 88.  What is left is the solve's
+// per pixel 138, and k_shade_visible 118 -> 84.  What is left is the solve's
 // arithmetic.  4 blocks of 128 per SM against 5 (some spilled) measured 151 and
 // 148 us before the divisions went, 6 157.
 template <bool Packed>
