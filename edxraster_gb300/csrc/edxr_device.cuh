@@ -578,7 +578,7 @@ __device__ __forceinline__ float3 shade_model(const FrameDesc& f, float3 P, floa
         if (f.ps_kind == 0)
             nh = fmaxf(nh, 0.0f);
         // nh^shininess as 2^(shininess log2 nh) (nh is clamped to >= 0 here:
-        // log2 0 = -inf gives 0; the unclamped reference shader shades in FP64)
+        // log2 0 = -inf gives 0; the unclamped reference shader shades in float pairs)
         spec = f.ks * exp2f(f.shininess * log2f(nh));
     }
     switch (f.ps_kind)
