@@ -1688,8 +1688,12 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
     // A pass of one frame (One) keeps its descriptor in shared memory: the
     // shading reads some twenty of its fields a pixel, and stores to the images
     // keep the compiler from holding them (raster stage: terrain 95 -> 93 us,
-    // binning stress 219 -> 211).
-    __shared__ FrameDesc s_frame;
+    // binning stress 219 -> 211).  With several frames each warp keeps its
+    // item's, copied when the frame changes: 256 views at 512x512 695 -> 678 us,
+    // 64 views at 256x256 110 -> 107.
+    __shared__ FrameDesc s_frames[One ? 1 : kRasterWarps];
+    FrameDesc& s_frame = s_frames[One ? 0 : threadIdx.x >> 5];
+    uint32_t in_shared = 0xFFFFFFFFu;  // several frames: the one whose descriptor the warp holds
     if (One)
         for (int k = (int)threadIdx.x; k < (int)(sizeof(FrameDesc) / 8); k += kRasterThreads)
             reinterpret_cast<unsigned long long*>(&s_frame)[k] = reinterpret_cast<const unsigned long long*>(a.frames)[k];
@@ -1724,12 +1728,15 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
     const uint32_t bulk = min(8u, max(1u, (nempty - shared_tiles) / ngroups));
     const uint32_t nwork = nitems + (nempty - shared_tiles + bulk - 1) / bulk;
     // the frame of a tile
+    auto frame_index = [&](uint32_t tile) -> uint32_t {
+        return a.tiles_per_frame ? tile / a.tiles_per_frame
+                                 : find_frame(a.frames, a.num_frames, tile,
+                                              [](const FrameDesc& f) { return f.tile_base; });
+    };
     auto frame_of = [&](uint32_t tile) -> const FrameDesc& {
         if (One)
             return s_frame;
-        return a.frames[a.tiles_per_frame ? tile / a.tiles_per_frame
-                                          : find_frame(a.frames, a.num_frames, tile,
-                                                       [](const FrameDesc& f) { return f.tile_base; })];
+        return a.frames[frame_index(tile)];
     };
     auto next_item = [&]() -> uint32_t {
         if (ngroups >= nwork)
@@ -1756,7 +1763,20 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
         for (uint32_t i = 0; i < share; i++)
             clear_tile(a, frame_of(a.empty_tiles[q * share + i]), a.empty_tiles[q * share + i], gthread, kThreads);
         const uint32_t tile = item.x & ~kSplitTile;
-        const FrameDesc& f = frame_of(tile);
+        if (!One)
+        {
+            const uint32_t fi = frame_index(tile);
+            if (fi != in_shared)
+            {
+                in_shared = fi;
+                __syncwarp();
+                for (uint32_t k = lane; k < sizeof(FrameDesc) / 8; k += 32)
+                    reinterpret_cast<unsigned long long*>(&s_frame)[k] =
+                        reinterpret_cast<const unsigned long long*>(a.frames + fi)[k];
+                __syncwarp();
+            }
+        }
+        const FrameDesc& f = s_frame;
         const uint32_t lt = tile - f.tile_base;
         const int tileX = (int)(lt % (uint32_t)f.tdx), tileY = (int)(lt / (uint32_t)f.tdx);
         const bool less = f.depth_func == 1;
