@@ -531,8 +531,8 @@ edxr_status launch_frames(edxr_renderer* r, uint32_t n, uint32_t width, uint32_t
     a.tiles_per_frame = equal_tiles && n > 1 ? (uint32_t)(tiles / n) : 0u;  // (one frame: no search)
     if (n > 1)
     {
-        EDXR_CUDA(r->frame_of_block.ensure(4 * (tt / 256 + 1)));
-        a.frame_of_block = r->frame_of_block.as<uint32_t>();
+        EDXR_CUDA(r->frame_of_block.ensure(sizeof(FrameHead) * (tt / 256 + 1)));
+        a.frame_of_block = r->frame_of_block.as<FrameHead>();
     }
     a.total_vertices = (uint32_t)tv;
     a.vrecs = vertex_stage ? r->vrecs.as<int4>() : nullptr;

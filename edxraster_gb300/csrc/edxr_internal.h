@@ -156,6 +156,17 @@ struct Tuning
 };
 
 // Launch parameters shared by every kernel of one pass.
+// The frame of a flattened input triangle and what setup needs first of it.
+struct __align__(16) FrameHead
+{
+    uint32_t frame;
+    uint32_t next_tri;   // the next frame's first triangle (~0: none)
+    uint32_t tri_base, vtx_base;
+    const uint32_t* indices;
+    uint32_t nv, pad;
+};
+static_assert(sizeof(FrameHead) == 32, "two 16-byte loads");
+
 struct PassArgs
 {
     Tuning tune;
@@ -163,7 +174,7 @@ struct PassArgs
     const FrameDesc* frames_host;  // page-locked: copied to `frames` at the start of the pass, or NULL
     uint32_t num_frames;
     uint32_t tiles_per_frame;  // every frame's tile count when they are equal (then frame = tile / it), else 0
-    uint32_t* frame_of_block;  // several frames: the frame of triangle 256 b, per b (filled by k_clear); else NULL
+    FrameHead* frame_of_block;  // several frames: of triangle 256 b, per b (filled by k_clear); else NULL
     uint32_t total_vertices;
     int4* vrecs;             // per flattened vertex: setup record (vertex stage), or NULL: setup projects in place
     uint32_t total_tris;
