@@ -198,13 +198,14 @@ struct PassArgs
     uint32_t big_capacity;
     uint32_t* counters;      // [0] fan-piece slots, [2] big tris, [3] raster work queue, [4] clip list,
                              // [6] heavy raster work items, [7] light ones, [8] scan block tickets,
-                             // [9] tiles with no bin entry,
+                             // [9] tiles with no bin entry, [10] the frame is dense (dense_entries),
                              // [11] surviving fan pieces, [kStripeBase + r * kStripeStride] stripe r of the
                              // unsorted bin list (kCounters words)
     unsigned long long* scan_status;  // per scan block (scan_blocks(total_tiles) words)
     uint4* items;            // raster work items (tile | split flag, first entry, end entry, the bin's start), one per
                              // item_entries-entry slice: heavy ones from the front, light ones from the back
     uint64_t item_capacity;
+    uint32_t dense_entries;  // a dense frame's item_entries, where the raster kernel is chosen by density; else 0
     uint32_t* empty_tiles;   // the tiles with no bin entry (counters[9] of them), total_tiles words
     unsigned long long* keybuf;  // per pixel: ~(smallest key) of split tiles, 0 between passes
     DeviceStatus* status;

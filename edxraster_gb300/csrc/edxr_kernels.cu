@@ -23,6 +23,7 @@ namespace edxr {
 constexpr int kRasterThreads = 256;    // 8 warps, each on its own work items
 constexpr uint32_t kBigChunk = 128;    // unsorted-list slots a k_bin_big warp reserves at a time
 constexpr uint32_t kEmptySlot = 0xFFFFFFFFu;
+constexpr uint32_t kDenseEntries = 640;  // entries a tile from which a frame is dense (see by_density)
 constexpr uint32_t kSplitTile = 0x80000000u;  // item tag: the tile has several items (tiles < 2^24)
 
 // Programmatic dependent launch: the pass's kernels follow one another with the
@@ -1095,7 +1096,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
     follow_on();
     __shared__ uint32_t warp_sums[33];
     __shared__ uint32_t s_block, s_prefix;
-    __shared__ bool s_dropped;
+    __shared__ bool s_dropped, s_dense;
     const uint32_t lane = threadIdx.x & 31;
     if (threadIdx.x == 0)
         s_block = atomicAdd(&a.counters[8], 1u);
@@ -1120,8 +1121,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
         filled = c[0];
         survived = c[1];
         const bool over = __any_sync(0xffffffffu, filled > stripe_slots(a.bin_capacity));
+        // many entries a tile: single warps rasterize them (see raster_group)
+        const bool dense = a.dense_entries && __reduce_add_sync(0xffffffffu, filled >> 4) >
+                                                  (uint64_t)a.total_tiles * (kDenseEntries >> 4);
         if (lane == 0)
+        {
             s_dropped = over;
+            s_dense = dense;
+            if (b == 0)
+                a.counters[10] = dense ? 1u : 0u;
+        }
     }
     uint32_t total;
     const uint32_t incl = block_scan(sum, warp_sums, total);
@@ -1179,7 +1188,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
     // reads a bin with missing entries or leaves a split tile's keys behind.
     const bool dropped = s_dropped;
     // entries per work item; items of at least 3/4 of that are heavy
-    const uint32_t E = (uint32_t)a.tune.item_entries, heavy_min = E - E / 4;
+    const uint32_t E = s_dense ? a.dense_entries : (uint32_t)a.tune.item_entries, heavy_min = E - E / 4;
     uint32_t run = prefix + incl - sum;
     uint32_t nheavy = 0, nlight = 0, nempty = 0;
     uint32_t start[kScanItems], n[kScanItems];
@@ -1699,6 +1708,8 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
     report_status(a);
     if (*(volatile uint32_t*)&a.status->error)
         return;  // the pass failed (see k_bin_move); every thread of the block leaves
+    if (a.dense_entries && (*(volatile uint32_t*)&a.counters[10] != 0) != (Group == 1))
+        return;  // the pass's other raster kernel takes the frame
     // ceil(65536 / w): ((p * s_recip[w]) >> 16) == p / w for 0 <= p < 256 and
     // 1 <= w <= 16, the row of pixel p of a region w pixels wide
     __shared__ uint32_t s_recip[17];
@@ -2720,6 +2731,20 @@ static int raster_group(const PassArgs& a, int sms)
     return tiles <= 30 * n || (tiles <= 60 * n && a.total_tris <= 120 * n) ? 4 : 1;
 }
 
+// Several warps rasterize an item's large regions together, each its own
+// pixels, so every warp looks at every one: where a tile has hundreds of
+// entries, most of them large, single warps are faster (raster stage,
+// several / one warp per item: 111,605 stress triangles at 427x394, 891 entries
+// a tile, 138 / 92 us; 30,000 at 320x180, 2,690 a tile, 66 / 53; but 10,000
+// there, 896 a tile, 51 / 49; the 1024x1024-quad terrain at 320x180, 543 a tile,
+// 27 / 40).  The entries are known after binning, so where the triangles allow
+// that many both kernels are launched, the scan decides and the other one
+// returns at once (1 us).
+static bool by_density(const PassArgs& a, int sms)
+{
+    return a.msaa_log2 == 0 && a.total_tris >= 64ull * a.total_tiles && raster_group(a, sms) > 1;
+}
+
 // Resident blocks per SM of k_raster_ms with 2^level samples (the dynamic
 // shared-memory limit raised first).
 template <int S>
@@ -2792,6 +2817,8 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
         // 113, 90 views at 300x200 96 / 92; 12 views there 25 / 30; the frames
         // of one mesh, terrain 92 / 103, binning stress 200 / 203).
         const bool many = a.num_frames > 1 && (uint64_t)a.total_tiles >= 96ull * (uint64_t)sms;
+        if (by_density(a, sms))
+            a.dense_entries = (uint32_t)a.tune.item_entries;
         a.tune.item_entries = min(1024, a.tune.item_entries * (many ? 2 : raster_group(a, sms)));
     }
     const uint32_t nscan = scan_blocks(a.total_tiles);
@@ -2851,6 +2878,8 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
         case 4: e = launch_raster<4>(sms, a, s, follows); break;
         default: e = launch_raster<1>(sms, a, s, follows); break;
         }
+        if (e == cudaSuccess && a.dense_entries)
+            e = launch_raster<1>(sms, a, s, follows);
     }
     mark(5);
     const cudaError_t last = cudaGetLastError();
@@ -2859,7 +2888,7 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
 
 int kernels_per_pass(const PassArgs& a)
 {
-    return 5 + (a.total_tris ? 2 : 0);
+    return 5 + (a.total_tris ? 2 : 0) + (by_density(a, a.num_sms > 0 ? a.num_sms : 148) ? 1 : 0);
 }
 
 __global__ void k_mip_level(const float4* src, int sw, int sh, float4* dst, int dw, int dh)
