@@ -2857,6 +2857,13 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
     if (a.msaa_log2 > 0)
     {
         const int level = min(a.msaa_log2, kMaxMsaaLog2), S = 1 << level;
+        // Not behind its predecessor's end (follow_on): blocks that become
+        // resident while others still run are placed under the shared-memory
+        // split those left, a few per SM, and as they stay until the work is
+        // done, the rest find no room (2 samples, 48,873 stress triangles at
+        // 164x125 427 -> 292 us a frame, 300,000 at 800x450 439 -> 350; terrain
+        // and sphere unchanged).
+        follows = false;
         const unsigned blocks = (unsigned)(sms * ms_occupancy(level)), threads = 32u * (unsigned)ms_warps(S);
         switch (level)
         {
