@@ -1121,7 +1121,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PassArgs a)
         filled = c[0];
         survived = c[1];
         const bool over = __any_sync(0xffffffffu, filled > stripe_slots(a.bin_capacity));
-        // many entries a tile: single warps rasterize them (see raster_group)
+        // many entries a tile: single warps rasterize them (see by_density; in
+        // sixteenths, so that the sum fits 32 bits)
         const bool dense = a.dense_entries && __reduce_add_sync(0xffffffffu, filled >> 4) >
                                                   (uint64_t)a.total_tiles * (kDenseEntries >> 4);
         if (lane == 0)
