@@ -1672,6 +1672,15 @@ __device__ __forceinline__ void report_status(const PassArgs& a)
         *a.status_host = *a.status;
 }
 
+// Entries a warp stages at a time when `warps` warps share n: the least that
+// takes as few rounds as chunks of 32 do, so that the last round is shared
+// evenly too.
+__device__ __forceinline__ uint32_t even_chunk(uint32_t n, uint32_t warps)
+{
+    const uint32_t rounds = (n + 32u * warps - 1u) / (32u * warps), shares = max(rounds, 1u) * warps;
+    return max(1u, (n + shares - 1u) / shares);
+}
+
 // Barrier of the Group warps that share an item: the warp's own lanes
 // (Group 1), the whole block (Group 8), or a named barrier per group.
 template <int Group>
@@ -1816,7 +1825,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
         uint32_t e0 = item.y, e1 = item.z, kept = 0;
         // entries a warp stages at a time: 32, fewer where not every warp of
         // the group would get some
-        const uint32_t per = Group == 1 ? 32u : min(32u, (e1 - e0 + (uint32_t)Group - 1u) / (uint32_t)Group);
+        const uint32_t per = Group == 1 ? 32u : even_chunk(e1 - e0, (uint32_t)Group);
         const uint32_t c0 = e0 + per * gwarp, cstep = per * (uint32_t)Group;
         uint32_t next = lane < per && c0 + lane < e1 ? a.bins[c0 + lane] : 0u;
         if (e0 != e1)
@@ -2480,7 +2489,7 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
         // entries a warp stages at a time: 32, fewer where all W would not get
         // some (100,000 stress triangles at 1920x1080, a handful of large ones
         // a tile: 8 samples 447 -> 326 us, 4 samples 296 -> 224)
-        const uint32_t per = min(32u, (e1 - e0 + (uint32_t)W - 1u) / (uint32_t)W);
+        const uint32_t per = even_chunk(e1 - e0, (uint32_t)W);
         for (uint32_t c = e0 + per * warp; c < e1; c += per * (uint32_t)W)
         {
             const uint32_t m = min(per, e1 - c);
