@@ -1673,11 +1673,11 @@ __device__ __forceinline__ void report_status(const PassArgs& a)
 }
 
 // Entries a warp stages at a time when `warps` warps share n: the least that
-// takes as few rounds as chunks of 32 do, so that the last round is shared
+// takes as few rounds as chunks of `most` do, so that the last round is shared
 // evenly too.
-__device__ __forceinline__ uint32_t even_chunk(uint32_t n, uint32_t warps)
+__device__ __forceinline__ uint32_t even_chunk(uint32_t n, uint32_t warps, uint32_t most = 32u)
 {
-    const uint32_t rounds = (n + 32u * warps - 1u) / (32u * warps), shares = max(rounds, 1u) * warps;
+    const uint32_t rounds = (n + most * warps - 1u) / (most * warps), shares = max(rounds, 1u) * warps;
     return max(1u, (n + shares - 1u) / shares);
 }
 
@@ -2384,6 +2384,7 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
     const uint32_t nitems = (uint32_t)min((uint64_t)nheavy + *(volatile uint32_t*)&a.counters[7], a.item_capacity);
     const uint64_t plane = a.total_pixels;
     const uint32_t nempty = *(volatile uint32_t*)&a.counters[9];
+    const bool dense = S <= 4 && *(volatile uint32_t*)&a.counters[10] != 0;
     const uint32_t bulk = min(8u, max(1u, nempty / gridDim.x));
     const uint32_t nwork = nitems + (nempty + bulk - 1) / bulk;
     // the items, then the tiles without an entry, as in k_raster
@@ -2488,8 +2489,13 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
         };
         // entries a warp stages at a time: 32, fewer where all W would not get
         // some (100,000 stress triangles at 1920x1080, a handful of large ones
-        // a tile: 8 samples 447 -> 326 us, 4 samples 296 -> 224)
-        const uint32_t per = even_chunk(e1 - e0, (uint32_t)W);
+        // a tile: 8 samples 447 -> 326 us, 4 samples 296 -> 224).  Of a dense
+        // frame's hundreds of entries a tile most lie behind the others: 16 at
+        // a time, so that the tile's bound is taken twice as often (4 samples,
+        // 100,000 stress triangles at 300x200 431 -> 336 us a frame, 215,347 at
+        // 216x129 656 -> 541, 845,117 at 271x229 1435 -> 1286; the
+        // 1024x1024-quad terrain at 320x180 185 -> 197)
+        const uint32_t per = even_chunk(e1 - e0, (uint32_t)W, dense ? 16u : 32u);
         for (uint32_t c = e0 + per * warp; c < e1; c += per * (uint32_t)W)
         {
             const uint32_t m = min(per, e1 - c);
@@ -2817,7 +2823,12 @@ cudaError_t launch_pipeline(const PassArgs& pass, cudaStream_t s, cudaEvent_t* e
     // more entries (twice, four times with 8 warps): 4 samples of the terrain
     // 309 -> 303 us, 16 samples 381 -> 317.
     if (a.msaa_log2 > 0)
+    {
         a.tune.item_entries = min(1024, a.tune.item_entries * (a.msaa_log2 <= 3 ? 2 : 4));
+        // (the items stay; k_raster_ms takes smaller chunks of a dense frame's)
+        if (a.msaa_log2 <= 2)
+            a.dense_entries = (uint32_t)a.tune.item_entries;
+    }
     else
     {
         // Several warps share an item; and with many small frames, four tiles
