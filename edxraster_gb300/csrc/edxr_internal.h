@@ -39,7 +39,8 @@ __host__ __device__ constexpr uint32_t scan_blocks(uint64_t tiles)
 // slots, each filled through its own counter (one 128-byte line apart, from
 // word kStripeBase of PassArgs::counters): word 0 the region's used slots,
 // word 1 the unclipped triangles that survived setup in warps of that
-// stripe (statistics).  Warps append to stripe (warp index mod kBinStripes),
+// stripe (statistics).  Warps append to stripe (warp index mod kBinStripes;
+// k_bin_big spreads the warps that share a triangle itself),
 // so no block-wide barrier is needed to keep one counter from being the
 // single address every warp of the grid contends for.
 constexpr int kBinStripes = 32;

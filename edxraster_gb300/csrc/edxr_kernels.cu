@@ -902,15 +902,26 @@ __device__ __forceinline__ uint32_t zmax_key(const RTri& t)
 // tiles does not leave lanes idle.  Each entry is counted in its tile and
 // kept in the unsorted list, which the warp fills from slots it reserves
 // kBigChunk at a time (one atomic on the shared counter per chunk); slots
-// it leaves unused are marked empty.
+// it leaves unused are marked empty.  Warps that share a triangle reserve what
+// a round needs and no more: a chunk for each of up to 32 warps would be up to
+// 4,096 slots for a thin triangle's hundred entries.
 __global__ void __launch_bounds__(256, 4) k_bin_big(PassArgs a)
 {
     follow_on();
     const uint32_t nb = min(*(volatile uint32_t*)&a.counters[2], a.big_capacity);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    // the warp's current chunk of its stripe of the unsorted list
-    const uint32_t stripe = warp_stripe();
+    // with few triangles, several warps share one, each taking every parts-th
+    // 32 of its tiles (a triangle over the whole screen is 7 rounds for one
+    // warp at 1366x769, 255 at 3840x2160)
+    const uint32_t parts = nb ? min(32u, max(1u, nw / nb)) : 1u;
+    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t group = gw / parts, part = gw % parts;
+    // the warp's current chunk of its stripe of the unsorted list: the stripes
+    // of a triangle's parts follow one another from its group's on, so that
+    // neither the parts of one triangle nor the first parts of all (the only
+    // ones with work where triangles have few tiles) meet in one stripe
+    const uint32_t stripe = (group + part) % (uint32_t)kBinStripes;
     const uint64_t send = stripe_begin(a, stripe) + stripe_slots(a.bin_capacity);
     uint64_t cbase = 0;
     uint32_t cleft = 0;
@@ -921,14 +932,8 @@ __global__ void __launch_bounds__(256, 4) k_bin_big(PassArgs a)
     };
     // batches of up to 32 triangles, small enough that every warp gets one
     const uint32_t batch = min(32u, max(1u, (nb + nw - 1) / nw));
-    // with few triangles, several warps share one, each taking every parts-th
-    // 32 of its tiles (a triangle over the whole screen is 7 rounds for one
-    // warp at 1366x769, 255 at 3840x2160)
-    const uint32_t parts = nb ? min(32u, max(1u, nw / nb)) : 1u;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int part = (int)(gw % parts);
     const bool early_cull = nb >= a.total_tiles;
-    for (uint32_t b0 = gw / parts * batch; b0 < nb; b0 += max(1u, nw / parts) * batch)
+    for (uint32_t b0 = group * batch; b0 < nb; b0 += max(1u, nw / parts) * batch)
     {
         // this lane's triangle of the batch and its number of 32x32 tiles
         uint32_t mine = kNoTriangle, mine_zocc = 0xFFFFFFFFu;
@@ -949,7 +954,7 @@ __global__ void __launch_bounds__(256, 4) k_bin_big(PassArgs a)
             if (lane >= (uint32_t)o) incl += v;
         }
         const int pairs = __shfl_sync(0xffffffffu, incl, 31);
-        for (int base = 32 * part; base < pairs; base += 32 * (int)parts)
+        for (int base = 32 * (int)part; base < pairs; base += 32 * (int)parts)
         {
             const int p = base + (int)lane;
             // owner: the first lane whose inclusive count exceeds p
@@ -1008,11 +1013,12 @@ __global__ void __launch_bounds__(256, 4) k_bin_big(PassArgs a)
             if (h > cleft)
             {
                 mark_empty();
+                const uint32_t chunk = parts > 1 ? h : kBigChunk;
                 uint32_t nbase = 0;
                 if (lane == 0)
-                    nbase = atomicAdd(stripe_counter(a, stripe), kBigChunk);
+                    nbase = atomicAdd(stripe_counter(a, stripe), chunk);
                 cbase = stripe_begin(a, stripe) + __shfl_sync(0xffffffffu, nbase, 0);
-                cleft = kBigChunk;
+                cleft = chunk;
             }
             uint64_t pos = cbase + (uint32_t)(cincl - cnt);
 #pragma unroll
