@@ -935,19 +935,22 @@ static __device__ __noinline__ float3 shade_fragment_fp64(const FrameDesc& f, co
     return f3(c, c, c);
 }
 
-// The same shader in float pairs (about 45 bits; Dekker 1971, Knuth): the
+// The same shader in float pairs (Dekker 1971, Knuth): the
 // FP64 unit issues a warp instruction every 16 cycles, and the 300 or so of
 // the FP64 form bounded the raster kernel (81 % of the FP64 unit busy).
-// Everything before the final rounding to float carries an error far below
-// float's, so the colours' error against 64 bits is the rounding's, as with
-// FP64.  Specular weights, exponents and N.H outside the plain range (see
-// `plain`) take the FP64 form.  256x256-quad terrain at 1280x720: a frame
-// 468 -> 127 us.
+// Each operation keeps about 45 bits, the logarithm and the exponential 38.  The
+// sums may cancel by a factor of 100, and a tilt of H is worth up to 6 sqrt(s)
+// times as much in the power where that is not lost in the diffuse term: within
+// the plain range (the two tests below; s <= 2048) the specular term is good to
+// 2^-28 at the worst and about 2^-35 as a rule, beside a rounding to float of
+// 2^-24.  Weights, exponents, vertices and N.H outside it take the FP64 form.
+// 256x256-quad terrain at 1280x720: a frame 468 -> 127 us.
 static __device__ __noinline__ float3 shade_fragment_pairs(const FrameDesc& f, const RTri* tg, const ClipPoly* polys,
                                                     float l0, float l1)
 {
+    if (!(fabsf(f.ks) <= 1e6f && f.shininess >= 0.0f && f.shininess <= 2048.0f))
+        return shade_fragment_fp64(f, tg, polys, l0, l1);
     const RTri t = load_rtri(tg);
-    const bool plain = fabsf(f.ks) <= 1e6f && f.shininess >= 0.0f && f.shininess <= 65536.0f;
     FF b[3] = { { l0, 0.0f }, { l1, 0.0f }, { 0.0f, 0.0f } };
     const FF rest = two_sum(1.0f, -l0);
     b[2] = ff_norm(ff_sum(rest, { -l1, 0.0f }));
@@ -959,6 +962,11 @@ static __device__ __noinline__ float3 shade_fragment_pairs(const FrameDesc& f, c
     b[1] = ff_div(b[1], sum);
     b[2] = ff_norm(ff_sum(ff_sum({ 1.0f, 0.0f }, ff_neg(b[0])), ff_neg(b[1])));
     const ShadeVerts v = shade_verts(f, t, polys);
+    // (for the plain range; here, while the vertices are at hand)
+    const float nmax = fmaxf(dot3(v.n[0], v.n[0]), fmaxf(dot3(v.n[1], v.n[1]), dot3(v.n[2], v.n[2])));
+    const float eye2 = dot3(f3(f.eye[0], f.eye[1], f.eye[2]), f3(f.eye[0], f.eye[1], f.eye[2]));
+    const float far2 = fmaxf(fmaxf(eye2, dot3(v.p[0], v.p[0])), fmaxf(dot3(v.p[1], v.p[1]), dot3(v.p[2], v.p[2])));
+    const float bmax = fmaxf(fabsf(b[0].hi), fmaxf(fabsf(b[1].hi), fabsf(b[2].hi)));
     FF E[3], N[3], L[3];
 #pragma unroll
     for (int q = 0; q < 3; q++)
@@ -986,19 +994,20 @@ static __device__ __noinline__ float3 shade_fragment_pairs(const FrameDesc& f, c
     const FF nh = ff_mul(ff_mul(ff_dot3(N, H), ninv), ff_rsqrt(h2));
     const float s = f.shininess, a = fabsf(nh.hi);
     // The plain range: no sum above cancelled by more than a factor of 100
-    // (10 bits of the 45), nothing near under- or overflow, and a power that
-    // exists (a negative N.H has one when the exponent is whole).
-    const float nmax = fmaxf(dot3(v.n[0], v.n[0]), fmaxf(dot3(v.n[1], v.n[1]), dot3(v.n[2], v.n[2])));
-    const float eye2 = dot3(f3(f.eye[0], f.eye[1], f.eye[2]), f3(f.eye[0], f.eye[1], f.eye[2]));
-    if (!(plain && a >= 1e-30f && a <= 2.0f && (nh.hi > 0.0f || s == rintf(s)) && n2.hi >= 1e-4f * nmax &&
-          n2.hi >= 1e-20f && n2.hi <= 1e20f && e2.hi >= 1e-4f * eye2 && e2.hi >= 1e-20f && e2.hi <= 1e20f &&
-          h2.hi >= 1e-4f && fabsf(sum.hi) >= 1e-15f && fabsf(sum.hi) <= 1e15f))
+    // (7 bits of the 45; the terms of P are weights times vertices, which may
+    // lie far beyond the pixel), nothing near under- or overflow, and a power
+    // that exists (a negative N.H has one when the exponent is whole).
+    if (!(a >= 1e-30f && a <= 2.0f && (nh.hi > 0.0f || s == rintf(s)) && n2.hi >= 1e-4f * nmax &&
+          n2.hi >= 1e-20f && n2.hi <= 1e20f && e2.hi >= 1e-4f * far2 && e2.hi >= 1e-20f &&
+          e2.hi <= 1e20f && bmax <= 2.0f && h2.hi >= 1e-4f && fabsf(sum.hi) >= 1e-15f && fabsf(sum.hi) <= 1e15f))
         return shade_fragment_fp64(f, tg, polys, l0, l1);
     const FF y = ff_norm(ff_prod_f(ff_log(nh.hi < 0.0f ? ff_neg(nh) : nh), s));
     FF spec = { 0.0f, 0.0f };
     if (y.hi > -80.0f)  // (below it the specular term is lost in the diffuse one's last bit)
         spec = ff_norm(ff_prod_f(ff_exp(y), nh.hi < 0.0f && ((int)s & 1) ? -f.ks : f.ks));
     const FF c = ff_norm(ff_sum(diffuse, spec));
+    if (!(fabsf(c.hi) >= 0.01f * diffuse.hi))  // (a specular term that takes the diffuse one away)
+        return shade_fragment_fp64(f, tg, polys, l0, l1);
     return f3(c.hi, c.hi, c.hi);
 }
 
