@@ -79,11 +79,14 @@ bool edxr::eye_from_mv(const float* mv, double eye[3])
     return true;
 }
 
-// v normalised in float, (1 / |v|) v with every operation rounded (kept in a
-// volatile: a host compiler may contract products and sums otherwise).
+// v normalised in float, (1 / |v|) v with every operation rounded.  The
+// products are formed in double, where they are exact, and rounded to float: a
+// host compiler contracts a float product and a sum otherwise.  (Stores to a
+// volatile did the same but cost 4 ns a frame, 2 % of a pass of 1,024 frames of
+// 32x32.)
 static void normalize_float(const float v[3], float unit[3], float& inv)
 {
-    auto mul = [](float a, float b) { volatile float r = a * b; return r; };
+    auto mul = [](float a, float b) { return (float)((double)a * (double)b); };
     const float x = mul(v[0], v[0]), y = mul(v[1], v[1]), z = mul(v[2], v[2]);
     const float len = std::sqrt((x + y) + z);
     inv = 1.0f / len;
