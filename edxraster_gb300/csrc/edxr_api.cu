@@ -133,8 +133,9 @@ void edxr::frame_mesh(FrameDesc& f, const edxr_mesh& m, uint32_t width, uint32_t
     f.uvs = static_cast<const char*>(m.uvs);
     f.indices = m.indices;
     f.pos_stride = m.position_stride;
-    f.nrm_stride = m.normal_stride;
-    f.alb_stride = m.albedo_stride;
+    // (an array that is missing: every vertex reads the one default, see copy_frame)
+    f.nrm_stride = m.normals ? m.normal_stride : 0u;
+    f.alb_stride = m.albedo ? m.albedo_stride : 0u;
     f.uv_stride = m.uv_stride;
     f.nv = m.num_vertices;
     f.nt = m.num_triangles;

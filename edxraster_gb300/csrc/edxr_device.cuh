@@ -492,18 +492,37 @@ __device__ __forceinline__ float3 normalize3(float3 v)
     const float inv = rsqrt_nr(dot3(v, v));
     return f3(v.x * inv, v.y * inv, v.z * inv);
 }
-// Element i of an array, `dflt` thrice where there is none (unless Present).
-template <bool Present = false>
-__device__ __forceinline__ float3 ld3(const char* base, uint32_t stride, uint32_t i, float dflt)
+__device__ __forceinline__ float3 ld3(const char* base, uint32_t stride, uint32_t i)
 {
-    if (!Present && !base)
-        return f3(dflt, dflt, dflt);
     const float* p = reinterpret_cast<const float*>(base + (size_t)i * stride);
     return f3(__ldg(p), __ldg(p + 1), __ldg(p + 2));
 }
 
-// Does the frame's mesh have every attribute array?
-__device__ __forceinline__ bool full_mesh(const FrameDesc& f) { return f.normals && f.albedo; }
+// What a vertex has of an attribute its mesh lacks: albedo 1, normal 0.
+static __device__ const float kNoAlbedo[3] = { 1.0f, 1.0f, 1.0f };
+static __device__ const float kNoNormal[3] = { 0.0f, 0.0f, 0.0f };
+
+// A frame's descriptor copied to shared memory by `threads` threads, for the
+// shading: arrays that the mesh lacks point to the one default (their stride is
+// 0).  Testing each of a pixel's nine loads for a missing array instead was
+// some 40 of its 350 instructions (raster stage: binning stress 210 -> 202 us,
+// terrain at 4 samples 238 -> 229).  A frame of the stress mesh without albedo,
+// 3840x2160: 378 us with the tests, 399 with such meshes shaded out of line, 370
+// now, as with albedo; the terrain at 8 samples 445, 455 and 416 (425).
+__device__ __forceinline__ void copy_frame(FrameDesc& to, const FrameDesc* from, uint32_t thread, uint32_t threads)
+{
+    static_assert(sizeof(FrameDesc) % 8 == 0 && offsetof(FrameDesc, normals) % 8 == 0 && offsetof(FrameDesc, albedo) % 8 == 0,
+                  "copied in words of 8 bytes");
+    for (uint32_t k = thread; k < sizeof(FrameDesc) / 8; k += threads)
+    {
+        unsigned long long w = reinterpret_cast<const unsigned long long*>(from)[k];
+        if (k == offsetof(FrameDesc, normals) / 8 && !w)
+            w = reinterpret_cast<unsigned long long>(kNoNormal);
+        if (k == offsetof(FrameDesc, albedo) / 8 && !w)
+            w = reinterpret_cast<unsigned long long>(kNoAlbedo);
+        reinterpret_cast<unsigned long long*>(&to)[k] = w;
+    }
+}
 
 // Per-pixel shading inputs of a triangle: its three vertices' position,
 // normal and albedo (after clipping) in object space.
@@ -514,21 +533,22 @@ struct ShadeVerts
 
 // Attributes of the raster vertices of triangle t (Clipper.h:138-151 for the
 // vertices the clipper created: weight.x*a0 + weight.y*a1 + weight.z*a2).
-// NormalsOnly: positions and albedo are not read (the textured shader).
-// Full: the mesh has normals and albedo (full_mesh); testing each of a pixel's
-// nine loads for a missing array was some 40 of its 350 instructions (raster
-// stage: binning stress 210 -> 202 us, terrain at 4 samples 238 -> 229).
-template <bool NormalsOnly = false, bool Full = false>
+// f is a copy_frame copy.  NormalsOnly: positions and albedo are not read (the
+// textured shader).
+template <bool NormalsOnly = false>
 __device__ __forceinline__ ShadeVerts shade_verts(const FrameDesc& f, const RTri& t, const ClipPoly* polys,
                                                   const uint32_t* vi = nullptr)
 {
     const uint32_t* idx = vi ? vi : f.indices + 3 * (size_t)(t.order >> 4);
-    const uint32_t i0 = vi ? vi[0] : __ldg(idx), i1 = vi ? vi[1] : __ldg(idx + 1), i2 = vi ? vi[2] : __ldg(idx + 2);
-    const char* pos = NormalsOnly ? nullptr : f.positions;
-    const char* alb = NormalsOnly ? nullptr : f.albedo;
-    float3 sp[3] = { ld3<Full>(pos, f.pos_stride, i0, 0.f), ld3<Full>(pos, f.pos_stride, i1, 0.f), ld3<Full>(pos, f.pos_stride, i2, 0.f) };
-    float3 sn[3] = { ld3<Full>(f.normals, f.nrm_stride, i0, 0.f), ld3<Full>(f.normals, f.nrm_stride, i1, 0.f), ld3<Full>(f.normals, f.nrm_stride, i2, 0.f) };
-    float3 sa[3] = { ld3<Full>(alb, f.alb_stride, i0, 1.f), ld3<Full>(alb, f.alb_stride, i1, 1.f), ld3<Full>(alb, f.alb_stride, i2, 1.f) };
+    const uint32_t i[3] = { vi ? vi[0] : __ldg(idx), vi ? vi[1] : __ldg(idx + 1), vi ? vi[2] : __ldg(idx + 2) };
+    float3 sp[3], sn[3], sa[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+    {
+        sp[k] = NormalsOnly ? f3(0.f, 0.f, 0.f) : ld3(f.positions, f.pos_stride, i[k]);
+        sn[k] = ld3(f.normals, f.nrm_stride, i[k]);
+        sa[k] = NormalsOnly ? f3(1.f, 1.f, 1.f) : ld3(f.albedo, f.alb_stride, i[k]);
+    }
     ShadeVerts v;
     if (t.poly == kUnclipped)
     {

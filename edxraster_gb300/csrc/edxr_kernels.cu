@@ -1524,7 +1524,6 @@ struct PixelOut
 // The per-vertex-attribute shaders (Blinn-Phong, Lambertian with or without
 // albedo) at barycentrics (L0, L1) of raster triangle t: perspective-correct
 // weights, the vertices' attributes, the shading model.  No call inside.
-template <bool Full>
 static __device__ __forceinline__ float3 shade_common(const FrameDesc& f, const RTri& t, const ClipPoly* polys,
                                                       float L0, float L1, const uint32_t* vi = nullptr)
 {
@@ -1537,25 +1536,14 @@ static __device__ __forceinline__ float3 shade_common(const FrameDesc& f, const 
     b0 = fmul(b0, invB);
     b1 = fmul(b1, invB);
     b2 = fsub(fsub(1.0f, b0), b1);
-    const ShadeVerts v = shade_verts<false, Full>(f, t, polys, vi);
+    const ShadeVerts v = shade_verts(f, t, polys, vi);
     return shade_model(f, lerp3(b0, v.p[0], b1, v.p[1], b2, v.p[2]), lerp3(b0, v.n[0], b1, v.n[1], b2, v.n[2]),
                        lerp3(b0, v.a[0], b1, v.a[1], b2, v.a[2]));
 }
 
 // Is the frame shaded out of line (the reference Blinn-Phong and the textured
-// shaders, and meshes without normals or albedo)?
-__device__ __forceinline__ bool slow_shading(const FrameDesc& f)
-{
-    return f.ps_kind == 1 || f.ps_kind == 4 || !full_mesh(f);
-}
-
-static __device__ __forceinline__ float3 shade_slow(const FrameDesc& f, const RTri& t, const RTri* tg,
-                                                    const ClipPoly* polys, float L0, float L1, int px, int py)
-{
-    if (f.ps_kind == 1 || f.ps_kind == 4)
-        return shade_fragment(f, t, tg, polys, L0, L1, px, py);
-    return shade_common<false>(f, t, polys, L0, L1);
-}
+// shaders)?
+__device__ __forceinline__ bool slow_shading(const FrameDesc& f) { return f.ps_kind == 1 || f.ps_kind == 4; }
 
 static __device__ __forceinline__ void write_pixel(const PixelOut a, const FrameDesc& f, uint32_t ri, uint64_t pix, int px,
                                                 int py)
@@ -1576,7 +1564,7 @@ static __device__ __forceinline__ void write_pixel(const PixelOut a, const Frame
     const float L1 = fmul(__int2float_rn(n2), t.invDet);
     const float L2 = fsub(fsub(1.0f, L0), L1);
     const float d = fadd(fadd(fmul(L0, t.z0), fmul(L1, t.z1)), fmul(L2, t.z2));
-    const float3 c = shade_slow(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
+    const float3 c = shade_fragment(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
     a.color[pix] = make_float4(c.x, c.y, c.z, 1.0f);
     a.depth[pix] = d;
     a.tri_id[pix] = t.order >> 4;
@@ -1601,15 +1589,15 @@ static __device__ __forceinline__ void write_pixel_fast(const PixelOut a, const 
     const RTri t = load_rtri(a.rtris + ri);
     float L0, L1;
     const float d = depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
-    const float3 c = shade_common<true>(f, t, a.polys, L0, L1, vi);
+    const float3 c = shade_common(f, t, a.polys, L0, L1, vi);
     a.color[pix] = make_float4(c.x, c.y, c.z, 1.0f);
     a.depth[pix] = d;
     a.tri_id[pix] = tri;
 }
 
-// A tile shaded by the reference Blinn-Phong or the textured shader or without
-// all of the attributes (slow_shading): out of line, pixel by
-// pixel, so that the common shaders' loop keeps its registers.
+// A tile shaded by the reference Blinn-Phong or the textured shader
+// (slow_shading): out of line, pixel by pixel, so that the common shaders' loop
+// keeps its registers.
 static __device__ __noinline__ void shade_tile_slow(const PixelOut out, const FrameDesc& f,
                                                     const unsigned long long* key, int first, int step, int tileX,
                                                     int tileY, bool less, uint32_t nr, const uint32_t* tri_first,
@@ -1739,8 +1727,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
     FrameDesc& s_frame = s_frames[One ? 0 : threadIdx.x >> 5];
     uint32_t in_shared = 0xFFFFFFFFu;  // several frames: the one whose descriptor the warp holds
     if (One)
-        for (int k = (int)threadIdx.x; k < (int)(sizeof(FrameDesc) / 8); k += kRasterThreads)
-            reinterpret_cast<unsigned long long*>(&s_frame)[k] = reinterpret_cast<const unsigned long long*>(a.frames)[k];
+        copy_frame(s_frame, a.frames, threadIdx.x, kRasterThreads);
     if (threadIdx.x >= 1 && threadIdx.x <= 16)
         s_recip[threadIdx.x] = (65536u + threadIdx.x - 1u) / threadIdx.x;
     __syncthreads();
@@ -1814,9 +1801,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassArgs a)
             {
                 in_shared = fi;
                 __syncwarp();
-                for (uint32_t k = lane; k < sizeof(FrameDesc) / 8; k += 32)
-                    reinterpret_cast<unsigned long long*>(&s_frame)[k] =
-                        reinterpret_cast<const unsigned long long*>(a.frames + fi)[k];
+                copy_frame(s_frame, a.frames + fi, lane, 32u);
                 __syncwarp();
             }
         }
@@ -2204,7 +2189,7 @@ __device__ __forceinline__ uint32_t to_byte(float v)
 // its busiest pixel (one to three) instead of once per sample at which any of
 // its pixels changes winner: 8 samples of the sphere at 1280x720, 94 -> 72 us.
 // The depth comes out of the key.  Common: the per-vertex-attribute shaders,
-// inline (no call); otherwise shade_slow (the reference and textured shaders
+// inline (no call); otherwise shade_fragment (the reference and textured shaders
 // out of line).
 template <int S, bool Common>
 static __device__ __forceinline__ void write_pixel_ms(const PassArgs& a, const FrameDesc& f,
@@ -2234,8 +2219,8 @@ static __device__ __forceinline__ void write_pixel_ms(const PassArgs& a, const F
             const RTri t = load_rtri(a.rtris + ri);
             float L0, L1;
             depth_at(t, (px << 4) + 8, (py << 4) + 8, L0, L1);
-            const float3 c = Common ? shade_common<true>(f, t, a.polys, L0, L1, vi)
-                                    : shade_slow(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
+            const float3 c = Common ? shade_common(f, t, a.polys, L0, L1, vi)
+                                    : shade_fragment(f, t, a.rtris + ri, a.polys, L0, L1, px, py);
             rgb = to_byte(c.x) | (to_byte(c.y) << 8) | (to_byte(c.z) << 16);
         }
 #pragma unroll (S <= 8 ? S : 4)
@@ -2371,8 +2356,7 @@ __global__ void __launch_bounds__(32 * ms_warps(S), ms_blocks(S)) k_raster_ms(co
     __shared__ uint32_t s_recip[17];
     // (several samples: one frame, its descriptor as in k_raster)
     __shared__ FrameDesc s_frame;
-    for (int k = (int)threadIdx.x; k < (int)(sizeof(FrameDesc) / 8); k += kThreads)
-        reinterpret_cast<unsigned long long*>(&s_frame)[k] = reinterpret_cast<const unsigned long long*>(a.frames)[k];
+    copy_frame(s_frame, a.frames, threadIdx.x, kThreads);
     const FrameDesc& f = s_frame;
     if (threadIdx.x >= 1 && threadIdx.x <= 16)
         s_recip[threadIdx.x] = (65536u + threadIdx.x - 1u) / threadIdx.x;
