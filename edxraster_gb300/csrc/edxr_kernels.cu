@@ -1625,18 +1625,6 @@ static __device__ __noinline__ void shade_tile_slow(const PixelOut out, const Fr
     }
 }
 
-
-// Key of a covered fragment from its two unbiased edge values; a NaN depth,
-// which never passes, gives ~0.
-__device__ __forceinline__ unsigned long long depth_key64(int l1, int l2, const StagedTri& s, uint32_t rank)
-{
-    const float L0 = fmul(__int2float_rn(l1), s.invDet);
-    const float L1 = fmul(__int2float_rn(l2), s.invDet);
-    const float L2 = fsub(fsub(1.0f, L0), L1);
-    const float d = fadd(fadd(fmul(L0, s.z0), fmul(L1, s.z1)), fmul(L2, s.z2));
-    return d == d ? ((unsigned long long)depth_key(d) << 32) | rank : ~0ull;
-}
-
 // The background of a tile, written by `threads` threads.
 static __device__ __forceinline__ void clear_tile(const PassArgs& a, const FrameDesc& f, uint32_t tile, int thread,
                                                   int threads)
