@@ -964,7 +964,7 @@ static __device__ __noinline__ float3 shade_fragment_fp64(const FrameDesc& f, co
 // the plain range (the two tests below; s <= 2048) the specular term is good to
 // 2^-28 at the worst and about 2^-35 as a rule, beside a rounding to float of
 // 2^-24.  Weights, exponents, vertices and N.H outside it take the FP64 form.
-// 256x256-quad terrain at 1280x720: a frame 468 -> 127 us.
+// 256x256-quad terrain at 1280x720, depth LEQUAL: a frame 675 -> 104 us.
 static __device__ __noinline__ float3 shade_fragment_pairs(const FrameDesc& f, const RTri* tg, const ClipPoly* polys,
                                                     float l0, float l1)
 {

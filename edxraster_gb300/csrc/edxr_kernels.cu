@@ -2326,7 +2326,9 @@ static __device__ __forceinline__ void clear_tile_ms(const PassArgs& a, const Fr
 // W and the blocks per SM (registers a thread): 4 warps at 8 blocks (64, some
 // spilled) against 5 (96, none) measured 270 and 313 us on the terrain at 4
 // samples, 55 and 51 on the sphere; 2 warps 291 and 59, 8 warps 350 and 61.
-// With 16 and 32 samples the keys allow 3 to 5 blocks: 8 warps each.
+// The shared memory (ms_smem) admits all 8 blocks up to 4 samples, 7 at 8
+// samples, 3 at 16 and 2 at 32: there 8 warps each.  The register caps are not
+// fitted to that (ms_blocks asks for 8 at 8 samples and 3 at 32).
 constexpr int kMsWarpBytes = 32 * (int)sizeof(StagedMs) + 64 * 2;
 
 __host__ __device__ constexpr int ms_warps(int S) { return S <= 8 ? 4 : 8; }

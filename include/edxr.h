@@ -292,7 +292,8 @@ typedef struct edxr_tuning
                                      many pixels are rasterized one triangle per thread; 0 disables */
     int raster_variant;           /* 0: one warp per raster work item; 1: one, or several where the
                                      frame has few tiles; 2: as 1, pixel-parallel only (small_region
-                                     ignored) */
+                                     ignored).  (0 and 1 once chose the registers of a kernel with one
+                                     warp per item, so a value stored then asks for another rule now.) */
     int bin_blocks_per_sm;        /* grid of the per-triangle binning kernels */
     int raster_blocks_per_sm;     /* persistent raster blocks per SM; 0 = the occupancy maximum */
     uint32_t bin_entries_per_triangle;  /* initial bin-buffer capacity per triangle (grows on overflow) */
